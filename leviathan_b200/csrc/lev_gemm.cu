@@ -8,16 +8,15 @@
 // weight rows into shared memory (bit-exact block decode, then one rounding to
 // bf16) and multiplies it against a slab of tokens.
 //
-// This first version issues mma.sync.m16n8k16 (bf16) from shared-memory tiles:
-// CTA tile 64 rows x 64 tokens, K-step 32, four warps of 32 x 32.  It is the
-// correctness anchor for the path; the tcgen05/TMEM mainloop replaces the
-// inner product without changing the operand rounding or the tile decode.
+// lev_gemm_pk.cu holds the tensor-memory kernel that serves the path.  The form here issues mma.sync.m16n8k16 (bf16)
+// from shared-memory tiles (CTA tile 64 rows x 64 tokens, K-step 32, four warps of 32 x 32) and serves what a TMA
+// load cannot: activations that do not start on a 16-byte boundary.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include "lev_internal.h"
 
-// tensor-memory form (lev_gemm_tc.cu)
+// tensor-memory form (lev_gemm_pk.cu)
 bool lev_gemm_tc_supported(const lev_weights* w, const void* x_bf16, int64_t tokens);
 int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int64_t tokens, float* y);
 

@@ -1,26 +1,5 @@
-// Prefill dequant-GEMM on the fifth-generation tensor cores (tcgen05 + TMEM), sm_100a.
-//
-//   Y[t][r] = sum_k bf16(W[r][k]) * X[t][k],  f32 accumulate in tensor memory
-//
-// Same operand rounding as the mma.sync form in lev_gemm.cu (weights decoded bit-exactly
-// as the block decoders form them, then one rounding to bf16; activations are bf16 already;
-// rust/crates/lev-forge/src/coopmat.rs:236-425, oracle rust/crates/lev-cli/src/main.rs:1201-1217).
-//
-// One CTA computes a tile of 256 tokens x 176 weight rows over the whole K:
-//   * warp 0 (one thread): TMA loads of the activation tile, two boxes of 128 tokens x 64 k
-//     (128-byte rows, hardware 128B swizzle) per K-step into a 3-stage ring;
-//   * warps 2..12 (352 threads): decode the K-step's 176 x 64 weights from the GGUF blocks in
-//     global memory and store them as bf16 into the same K-major 128B-swizzled layout, then
-//     publish them to the async proxy (fence.proxy.async) and arrive on the stage's barrier;
-//   * warp 1 (one thread): for each K-step 4 x 2 tcgen05.mma (M = 128 tokens, N = 176 rows,
-//     K = 16) from shared-memory descriptors into two TMEM accumulators (352 of 512 columns),
-//     tcgen05.commit hands the stage back to the producers;
-//   * epilogue: warps 2..9 read the accumulators with tcgen05.ld (warp w owns TMEM lanes
-//     32*(w%4)...) and store Y rows with 16-byte stores.
-// Decode batches (up to 128 tokens) of the 4-bit formats take the STAGED form of the same kernel: the raw
-// bytes reach shared memory by cp.async one 256-column group ahead and two threads share a weight row; the
-// launch then also splits K over gridDim.z, partial products summed in split order by k_gemm_split_sum.
-// The grouped forms further down serve the routed MoE (weights as the MMA's M operand).
+// Grouped dequant-GEMM of the routed MoE at prefill-sized token counts (tcgen05 + TMEM), sm_100a: the weight rows of an
+// expert are the MMA's M, the tokens routed to it its N.  The dense GEMM is lev_gemm_pk.cu.
 // Every wait is bounded by about a second of SM clocks; on a timeout the CTA sets
 // LEV_DEV_TIMEOUT, skips the remaining work, frees its tensor memory and returns.
 #include <cuda.h>
@@ -33,31 +12,10 @@
 
 namespace {
 
-constexpr int TM = 256;      // tokens per CTA tile (two MMA tiles of 128)
-constexpr int RN = 176;      // weight rows per CTA tile (MMA N): 12288 rows x 512 tokens -> 140 CTAs on 148 SMs
 constexpr int KS = 64;       // k per pipeline stage (one 128-byte swizzle row of bf16)
-constexpr int STAGES = 3;
-constexpr int kDequantWarps = 11;
-constexpr int kThreads = (2 + kDequantWarps) * 32;
-constexpr int kXHalfBytes = 128 * KS * 2;             // 16384: one TMA box
-constexpr int kXStageBytes = 2 * kXHalfBytes;         // 32768
-constexpr int kWStageBytes = RN * KS * 2;             // 24576
-constexpr int kStageBytes = kXStageBytes + kWStageBytes;
-constexpr int kTmemCols = 512;
+constexpr int kXHalfBytes = 128 * KS * 2;             // one TMA box of 128 tokens
 constexpr long long kWaitCycles = 2000000000LL;
 constexpr int kAhead = 3;  // K-steps of raw weight bytes a decode thread has requested ahead of the one it decodes
-
-struct GemmTcArgs {
-    const uint8_t* raw;   // GGUF blocks, row-major
-    int type;
-    int64_t row_bytes;
-    int64_t rows, cols;
-    int tokens;
-    float* y;             // [tokens][rows]; with a K split: [gridDim.z][tokens][rows] partial products
-    int y_vec;            // rows of y start on 16-byte boundaries
-    int* status;
-    int ksteps_per_split; // K-steps a CTA takes (blockIdx.z picks the range); the whole K without a split
-};
 
 __device__ __forceinline__ unsigned s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ float h2f(unsigned bits) { return __half2float(__ushort_as_half((unsigned short)bits)); }
@@ -106,15 +64,6 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
 // shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t umma_desc(unsigned smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// instruction descriptor: D f32, A and B bf16, both K-major, M = 128, N = RN
-constexpr unsigned kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(RN >> 3) << 17) | ((unsigned)(128 >> 4) << 24);
-
-__device__ __forceinline__ void umma_bf16(unsigned d_tmem, uint64_t adesc, uint64_t bdesc, unsigned accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(kInstrDesc), "r"(accumulate)
-        : "memory");
 }
 __device__ __forceinline__ void umma_commit(unsigned bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar) : "memory");
@@ -287,314 +236,6 @@ __device__ __forceinline__ void decode_store(const RowRaw<TYPE>& R, int it, int 
     }
     *reinterpret_cast<uint4*>(wtile + swz(r, ch_lo)) = pack8(lo);
     *reinterpret_cast<uint4*>(wtile + swz(r, ch_hi)) = pack8(hi);
-}
-
-// ---- staged decode of the dense kernel: two threads per weight row ----
-// The raw GGUF bytes of the tile's 176 rows x 256 columns (144 bytes per row for both 4-bit formats) are copied
-// to shared memory by cp.async one group ahead; a thread reads its row's bytes with 16-byte shared loads (rows
-// 144 bytes apart: eight lanes cover the 32 banks) and produces 32 of the K-step's 64 values, four 16-byte chunks
-// of the swizzled tile row.  Thread half h takes the low (0) or the high (1) nibbles, so both halves run the
-// same instructions with a shift of 4h.
-constexpr int DS_ROW_BYTES = 144;
-constexpr int DS_RAW_BYTES = RN * DS_ROW_BYTES;     // 25344 per group
-constexpr int kDecodeThreads = kDequantWarps * 32;   // 352 = 2 x RN
-static_assert(kDecodeThreads == 2 * RN && DS_RAW_BYTES % 16 == 0, "two decode threads per weight row");
-__device__ __forceinline__ void dense_decode_barrier() { asm volatile("bar.sync 1, %0;\n" ::"n"(kDecodeThreads) : "memory"); }
-
-// Q4_K: K-step c of the block whose 144 bytes start at blk; half h = sub-block 2c + h.  value = d1 * q - m1 with
-// d1 = d * sc, m1 = dmin * m as the reference forms them (rust/crates/lev-cpu/src/lib.rs:110-130); d1 * q is
-// exact in f32 (11 + 6 + 4 bits), so the fused multiply-add gives the bits of its multiply-then-subtract.
-__device__ __forceinline__ void q4k_half_store(const unsigned char* blk, int c, unsigned h, unsigned char* wtile, int r) {
-    const uint4 hdr = *reinterpret_cast<const uint4*>(blk);
-    const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + 32 * c), qb = *reinterpret_cast<const uint4*>(blk + 32 + 32 * c);
-    const float d = h2f(hdr.x & 0xffffu), dmin = h2f(hdr.x >> 16);
-    const unsigned sc_w = c < 2 ? (hdr.y & 0x3F3F3F3Fu) : ((hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u));
-    const unsigned mn_w = c < 2 ? (hdr.z & 0x3F3F3F3Fu) : (((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u));
-    const unsigned sh = 8u * (2u * (unsigned)(c & 1) + h);
-    const float d1 = __fmul_rn(d, (float)((sc_w >> sh) & 0xffu)), nm1 = -__fmul_rn(dmin, (float)((mn_w >> sh) & 0xffu));
-    const unsigned w[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        float v[8];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const unsigned n4 = (w[2 * j + k] >> (4u * h)) & 0x0F0F0F0Fu;
-#pragma unroll
-            for (int i = 0; i < 4; i++) v[4 * k + i] = __fmaf_rn(d1, __uint_as_float(__byte_perm(n4, 0x4B000000u, 0x7650u + i)) - 8388608.0f, nm1);
-        }
-        *reinterpret_cast<uint4*>(wtile + swz(r, 4 * (int)h + j)) = pack8(v);
-    }
-}
-
-// Q4_0: K-step S (0..3) of a 256-column group = the two blocks at byte 36 * S of the row's 144; half h takes the
-// low or high nibbles of both blocks: values 16h .. 16h + 15 of each, chunks 4b + 2h and 4b + 2h + 1.
-// d * (128 + q) - 136 d is exact and equals the reference's d * (q - 8) (Sources/LeviathanCore/Q4.swift:54-69).
-template <int S>
-__device__ __forceinline__ void q40_half_store(const unsigned char* rowraw, unsigned h, unsigned char* wtile, int r) {
-    const uint4* src = reinterpret_cast<const uint4*>(rowraw + ((36 * S) & ~15));
-    unsigned L[12];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const uint4 v4 = src[c];
-        L[4 * c] = v4.x; L[4 * c + 1] = v4.y; L[4 * c + 2] = v4.z; L[4 * c + 3] = v4.w;
-    }
-    const unsigned* w = L + S;   // the 36 bytes start at word S of the window
-#pragma unroll
-    for (int b = 0; b < 2; b++) {
-        unsigned q[4];
-        unsigned dbits;
-        if (b == 0) {
-            dbits = w[0] & 0xffffu;
-#pragma unroll
-            for (int k = 0; k < 4; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 16);
-        } else {
-            dbits = w[4] >> 16;
-#pragma unroll
-            for (int k = 0; k < 4; k++) q[k] = w[5 + k];
-        }
-        const float d = h2f(dbits), c136 = __fmul_rn(d, -136.0f);
-#pragma unroll
-        for (int j = 0; j < 2; j++) {
-            float v[8];
-#pragma unroll
-            for (int k = 0; k < 2; k++) {
-                const unsigned n4 = (q[2 * j + k] >> (4u * h)) & 0x0F0F0F0Fu;
-#pragma unroll
-                for (int i = 0; i < 4; i++) v[4 * k + i] = __fmaf_rn(d, __uint_as_float(__byte_perm(n4, 0x43000000u, 0x7054u + (i << 8))), c136);
-            }
-            *reinterpret_cast<uint4*>(wtile + swz(r, 4 * b + 2 * (int)h + j)) = pack8(v);
-        }
-    }
-}
-
-template <int TYPE, bool STAGED>
-__global__ void __launch_bounds__(kThreads, 1) k_gemm_tc(const __grid_constant__ CUtensorMap xmap, GemmTcArgs A) {
-    extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long full_x[STAGES], full_w[STAGES], empty[STAGES], accum_full;
-    __shared__ unsigned tmem_base_s;
-    __shared__ int abort_s;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // the swizzled tiles need 1024-byte alignment
-    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-    const int64_t r0 = (int64_t)blockIdx.x * RN;
-    const int t0 = blockIdx.y * TM;
-    const int halves = A.tokens - t0 > 128 ? 2 : 1;
-    // K split: this CTA's K-steps are [kbase, kbase + kt) of the tensor's, its output slab is blockIdx.z
-    const int kt_all = (int)(A.cols / KS);
-    const int kbase = (int)blockIdx.z * A.ksteps_per_split;
-    const int kt = kt_all - kbase < A.ksteps_per_split ? kt_all - kbase : A.ksteps_per_split;
-    float* const yout = A.y + (int64_t)blockIdx.z * A.tokens * A.rows;
-
-    if (threadIdx.x == 0) {
-        abort_s = 0;
-        for (int s = 0; s < STAGES; s++) {
-            mbar_init(s32(&full_x[s]), 1);
-            mbar_init(s32(&full_w[s]), kDequantWarps);
-            mbar_init(s32(&empty[s]), 1);
-        }
-        mbar_init(s32(&accum_full), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(s32(&tmem_base_s)), "r"(kTmemCols)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const unsigned tmem_base = tmem_base_s;
-    volatile int* abort_flag = &abort_s;
-
-    if (warp == 0) {
-        // ---- activation tiles by TMA ----
-        if (lane == 0) {
-            for (int it = 0; it < kt; it++) {
-                const int s = it % STAGES;
-                if (it >= STAGES && !mbar_wait(s32(&empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag)) break;
-                const unsigned dst = s32(smem + (size_t)s * kStageBytes);
-                mbar_expect_tx(s32(&full_x[s]), halves * kXHalfBytes);
-                tma_load_2d(dst, &xmap, (kbase + it) * KS, t0, s32(&full_x[s]));
-                if (halves == 2) tma_load_2d(dst + kXHalfBytes, &xmap, (kbase + it) * KS, t0 + 128, s32(&full_x[s]));
-            }
-        }
-    } else if (warp == 1) {
-        // ---- MMA issue ----
-        if (lane == 0) {
-            bool ok = true;
-            for (int it = 0; it < kt && ok; it++) {
-                const int s = it % STAGES;
-                const unsigned ph = (it / STAGES) & 1;
-                ok = mbar_wait(s32(&full_x[s]), ph, abort_flag);
-                ok = ok && mbar_wait(s32(&full_w[s]), ph, abort_flag);
-                if (!ok) break;
-                asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const unsigned xs = s32(smem + (size_t)s * kStageBytes), ws = xs + kXStageBytes;
-#pragma unroll
-                for (int kk = 0; kk < KS / 16; kk++) {
-                    const uint64_t bdesc = umma_desc(ws + kk * 32);
-                    for (int h = 0; h < halves; h++)
-                        umma_bf16(tmem_base + h * RN, umma_desc(xs + h * kXHalfBytes + kk * 32), bdesc, (it | kk) ? 1u : 0u);
-                }
-                umma_commit(s32(&empty[s]));  // the stage may be refilled when these MMAs have read it
-            }
-            umma_commit(s32(&accum_full));
-        }
-    } else {
-        bool ok = true;
-        if constexpr (STAGED) {
-            // ---- weight staging and decode: thread = (weight row, nibble half) ----
-            const int dt = threadIdx.x - 64;
-            const int row = dt % RN;
-            const unsigned half_h = (unsigned)(dt / RN);
-            unsigned char* rawbuf = smem + (size_t)STAGES * kStageBytes;
-            const int ngroups = kt >> 2;              // this form serves K in whole 256-column groups
-            // decode warp dw stages rows dw, dw + 11, ... (16 rows): lanes 0..26 take three rows at a time, nine
-            // 16-byte pieces each
-            const int dw = warp - 2;
-            const int l9 = lane / 9, p9 = lane - 9 * l9;
-            auto stage_group = [&](int g) {
-                const unsigned dst0 = s32(rawbuf + (size_t)(g & 1) * DS_RAW_BYTES);
-                const uint8_t* src0 = A.raw + r0 * A.row_bytes + (int64_t)((kbase >> 2) + g) * DS_ROW_BYTES;
-                if (lane < 27) {
-#pragma unroll
-                    for (int q = 0; q < 6; q++) {
-                        const int m = 3 * q + l9;
-                        const int r = dw + kDequantWarps * m;
-                        if (m < 16 && r0 + r < A.rows) cp_async16(dst0 + r * DS_ROW_BYTES + p9 * 16, src0 + (int64_t)r * A.row_bytes + p9 * 16);
-                    }
-                }
-            };
-            if (ngroups > 0) stage_group(0);
-            cp_async_commit();
-            for (int g = 0; g < ngroups; g++) {
-                cp_async_wait_but<0>();       // this thread's copies of group g have landed
-                dense_decode_barrier();       // everyone's have, and everyone is done reading the other slot
-                if (g + 1 < ngroups && ok) stage_group(g + 1);
-                cp_async_commit();
-                const unsigned char* rowraw = rawbuf + (size_t)(g & 1) * DS_RAW_BYTES + row * DS_ROW_BYTES;
-                auto kstep = [&](auto s_tag) {
-                    constexpr int SK = decltype(s_tag)::value;
-                    const int it = 4 * g + SK;
-                    if (!ok) return;
-                    const int s = it % STAGES;
-                    if (it >= STAGES) ok = mbar_wait(s32(&empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag);
-                    if (!ok) return;
-                    unsigned char* wtile = smem + (size_t)s * kStageBytes + kXStageBytes;
-                    if (TYPE == LEV_GGML_Q4_K) q4k_half_store(rowraw, SK, half_h, wtile, row);
-                    else q40_half_store<SK>(rowraw, half_h, wtile, row);
-                    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic stores -> visible to the tensor core's reads
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(s32(&full_w[s]));
-                };
-                kstep(std::integral_constant<int, 0>());
-                kstep(std::integral_constant<int, 1>());
-                kstep(std::integral_constant<int, 2>());
-                kstep(std::integral_constant<int, 3>());
-            }
-            cp_async_wait_but<0>();
-        } else {
-        // ---- weight decode: thread = (2 rows 88 apart) x (byte group j); the raw bytes of the
-        // next K-step are requested before this one is decoded ----
-        // lanes 0..7 of a warp take byte group 0 of eight consecutive rows, lanes 8..15 group 1, ...:
-        // the eight 16-byte stores of one shared-memory wavefront then fall into eight different
-        // bank groups of the swizzled tile
-        const int j = lane >> 3, rb = (warp - 2) * 8 + (lane & 7);
-        constexpr int kRowStep = kDequantWarps * 8;   // rows covered by one pass of the decode threads
-        constexpr int NR = RN / kRowStep;
-        static_assert(RN % kRowStep == 0, "decode threads tile the weight rows evenly");
-        RowRaw<TYPE> ahead[kAhead][NR];
-        const uint8_t* rowp[NR];
-        bool valid[NR];
-#pragma unroll
-        for (int i = 0; i < NR; i++) {
-            valid[i] = r0 + rb + kRowStep * i < A.rows;
-            rowp[i] = A.raw + (r0 + (valid[i] ? rb + kRowStep * i : 0)) * A.row_bytes;
-#pragma unroll
-            for (int u = 0; u < kAhead; u++)
-                if (u < kt) load_raw<TYPE>(rowp[i], kbase + u, j, valid[i], ahead[u][i]);
-        }
-        for (int it0 = 0; it0 < kt && ok; it0 += kAhead) {
-#pragma unroll
-            for (int u = 0; u < kAhead; u++) {
-                const int it = it0 + u;
-                if (it >= kt || !ok) break;
-                const int s = it % STAGES;
-                RowRaw<TYPE> cur[NR];
-#pragma unroll
-                for (int i = 0; i < NR; i++) {
-                    cur[i] = ahead[u][i];
-                    if (it + kAhead < kt) load_raw<TYPE>(rowp[i], kbase + it + kAhead, j, valid[i], ahead[u][i]);
-                }
-                if (it >= STAGES) ok = mbar_wait(s32(&empty[s]), ((it / STAGES) & 1) ^ 1, abort_flag);
-                if (!ok) break;
-                unsigned char* wtile = smem + (size_t)s * kStageBytes + kXStageBytes;
-#pragma unroll
-                for (int i = 0; i < NR; i++) decode_store<TYPE>(cur[i], kbase + it, j, valid[i], wtile, rb + kRowStep * i);
-                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // generic stores -> visible to the tensor core's reads
-                __syncwarp();
-                if (lane == 0) mbar_arrive(s32(&full_w[s]));
-            }
-        }
-        }
-        // ---- epilogue: TMEM -> Y ----
-        if (ok && warp < 10 && mbar_wait(s32(&accum_full), 0, abort_flag)) {
-            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            const int quarter = warp & 3, half = (warp - 2) >> 2;
-            if (half < halves) {
-                unsigned* stg = reinterpret_cast<unsigned*>(smem) + (warp - 2) * (32 * 36);
-#pragma unroll 1
-                for (int c = 0; c < RN; c += 32) {
-                    unsigned v[32];
-                    const unsigned taddr = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)(half * RN + c);
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-                          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-                          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-                          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                        : "r"(taddr)
-                        : "memory");
-                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                    // transpose through shared memory (the pipeline stages are idle now) so that every
-                    // store instruction writes whole 128-byte lines of four token rows
-                    __syncwarp();
-#pragma unroll
-                    for (int q = 0; q < 32; q += 4)
-                        *reinterpret_cast<uint4*>(stg + lane * 36 + q) = make_uint4(v[q], v[q + 1], v[q + 2], v[q + 3]);
-                    __syncwarp();
-                    const int col4 = (lane & 7) * 4;
-#pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int tl = i * 4 + (lane >> 3);
-                        const int tok = t0 + half * 128 + quarter * 32 + tl;
-                        const uint4 o = *reinterpret_cast<const uint4*>(stg + tl * 36 + col4);
-                        if (tok < A.tokens && c + col4 < RN) {  // the last chunk of a tile may be narrower than 32
-                            float* dst = yout + (int64_t)tok * A.rows + r0 + c + col4;
-                            if (r0 + c + col4 + 4 <= A.rows && A.y_vec) {
-                                *reinterpret_cast<uint4*>(dst) = o;
-                            } else {
-                                const unsigned ov[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-                                for (int q = 0; q < 4; q++)
-                                    if (r0 + c + col4 + q < A.rows) dst[q] = __uint_as_float(ov[q]);
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-    if (abort_s && threadIdx.x == 0) atomicOr(A.status, LEV_DEV_TIMEOUT);
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1200,109 +841,7 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-// y = sum over the K splits' partial products, in split order (the same bits on every run)
-__global__ void __launch_bounds__(256) k_gemm_split_sum(const float4* __restrict__ part, int splits, int64_t n4, float4* __restrict__ y) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 a = part[i];
-        for (int z = 1; z < splits; z++) {
-            const float4 b = part[(int64_t)z * n4 + i];
-            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-        }
-        y[i] = a;
-    }
-}
-
-template <int TYPE, bool STAGED>
-int launch_tc(lev_ctx* ctx, const CUtensorMap& map, const GemmTcArgs& A, dim3 grid, size_t smem) {
-    static bool configured[16] = {};
-    if (!configured[ctx->device & 15]) {
-        LEV_CUDA(ctx, cudaFuncSetAttribute(k_gemm_tc<TYPE, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured[ctx->device & 15] = true;
-    }
-    k_gemm_tc<TYPE, STAGED><<<grid, kThreads, smem, ctx->stream>>>(map, A);
-    return LEV_OK;
-}
-
 }  // namespace
-
-// shapes the tensor-memory kernel serves: rows whose K is a multiple of 64,
-// 16-byte aligned activations
-bool lev_gemm_tc_supported(const lev_weights* w, const void* x_bf16, int64_t tokens) {
-    if (w->type != LEV_GGML_Q4_K && w->type != LEV_GGML_Q4_0 && w->type != LEV_GGML_Q6_K) return false;
-    if (w->cols % KS != 0 || ((uintptr_t)x_bf16 & 15) != 0 || tokens < 1) return false;
-    return encode_tiled() != nullptr;
-}
-
-int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int64_t tokens, float* y) {
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return lev_fail(ctx, LEV_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
-    CUtensorMap map;
-    const cuuint64_t gdim[2] = {(cuuint64_t)w->cols, (cuuint64_t)tokens};
-    const cuuint64_t gstride[1] = {(cuuint64_t)w->cols * 2};
-    const cuuint32_t box[2] = {KS, 128};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(x_bf16), gdim, gstride, box, estr,
-                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) return lev_fail(ctx, LEV_KERNEL_FAILED, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
-    GemmTcArgs A;
-    A.raw = w->raw;
-    A.type = w->type;
-    A.row_bytes = w->blocks_per_row * lev_block_bytes(w->type);
-    A.rows = w->rows;
-    A.cols = w->cols;
-    A.tokens = (int)tokens;
-    A.y = y;
-    A.y_vec = ((uintptr_t)y & 15) == 0 && (w->rows & 3) == 0;
-    A.status = ctx->d_status;
-    A.ksteps_per_split = (int)(w->cols / KS);
-    dim3 grid((unsigned)((w->rows + RN - 1) / RN), (unsigned)((tokens + TM - 1) / TM));
-    const size_t smem = (size_t)STAGES * kStageBytes + 1024;
-    // Up to 128 tokens (decode batches) the kernel is bound by the weight decode: the 4-bit formats then decode from
-    // raw bytes staged in shared memory (40 % fewer instructions), when K comes in whole 256-column groups and every
-    // row starts on a 16-byte boundary (16-byte asynchronous copies).  Above that the token tiles' trip from L2 is
-    // the bound (measured: decode warps wait on the MMA's stage release 45 % of the time) and the register-staged
-    // form, which leaves shared memory to the pipeline, is the faster one (73 against 80 us on 512 x 12288 x 4096).
-    const bool staged = tokens <= 128 && w->type != LEV_GGML_Q6_K && w->cols % 256 == 0 && A.row_bytes % 16 == 0 &&
-                        ((uintptr_t)A.raw & 15) == 0;
-    const size_t smem_staged = smem + 2 * (size_t)DS_RAW_BYTES;
-    // A decode batch against a tensor of a few thousand rows makes a few dozen tiles, each a serial walk over the
-    // whole K: split K over gridDim.z (whole 256-column groups) until the SMs are covered, partial products to
-    // scratch, summed in split order by a second launch.
-    int splits = 1;
-    const int64_t groups = w->cols / 256, tiles = (int64_t)grid.x * grid.y;
-    const bool can_sum = ((uintptr_t)y & 15) == 0 && (tokens * w->rows) % 4 == 0;
-    if (staged && can_sum && tiles * 2 <= ctx->prop.multiProcessorCount && groups >= 2) {
-        int64_t want = ctx->prop.multiProcessorCount / tiles;
-        if (want > 8) want = 8;
-        if (want > groups) want = groups;
-        const int64_t per = (groups + want - 1) / want;          // groups per split
-        splits = (int)((groups + per - 1) / per);
-        A.ksteps_per_split = (int)(4 * per);
-    }
-    float* y_final = y;
-    if (splits > 1) {
-        void* scr;
-        LEV_TRY(lev_scratch(ctx, LEV_SCR_GEMM, (size_t)splits * tokens * w->rows * sizeof(float), &scr));
-        A.y = (float*)scr;
-        grid.z = (unsigned)splits;
-    }
-    int st = w->type == LEV_GGML_Q6_K ? launch_tc<LEV_GGML_Q6_K, false>(ctx, map, A, grid, smem)
-             : w->type == LEV_GGML_Q4_K
-                 ? (staged ? launch_tc<LEV_GGML_Q4_K, true>(ctx, map, A, grid, smem_staged) : launch_tc<LEV_GGML_Q4_K, false>(ctx, map, A, grid, smem))
-                 : (staged ? launch_tc<LEV_GGML_Q4_0, true>(ctx, map, A, grid, smem_staged) : launch_tc<LEV_GGML_Q4_0, false>(ctx, map, A, grid, smem));
-    if (st) return st;
-    ctx->launches++;
-    LEV_TRY(lev_cuda_check(ctx, cudaGetLastError(), "k_gemm_tc"));
-    if (splits > 1) {
-        const int64_t n4 = tokens * w->rows / 4;
-        int64_t blocks = (n4 + 255) / 256, cap = (int64_t)ctx->prop.multiProcessorCount * 4;
-        k_gemm_split_sum<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, ctx->stream>>>((const float4*)A.y, splits, n4, (float4*)y_final);
-        ctx->launches++;
-        return lev_cuda_check(ctx, cudaGetLastError(), "k_gemm_split_sum");
-    }
-    return LEV_OK;
-}
 
 // ---------------------------------------------------------------------------
 // grouped form: host side

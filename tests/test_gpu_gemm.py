@@ -60,3 +60,27 @@ def test_gemm_rejections(ctx):
         ctx._check(ctx.lib.lev_gemm_prefill(ctx.handle, wh.handle, 1, 0, 1, 0))
     assert e.value.name == "badDimensions"
     wh.free()
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q4_k", "q6_k"])
+@pytest.mark.parametrize("rows,cols,tokens", [
+    (16, 256, 17),       # one 16-row tile of eight, a second N step of 16
+    (272, 1280, 129),    # first size of the CTA pairs: the last pair's second CTA has no rows; five K-steps of 256
+    (250, 768, 288),     # two MMAs side by side, a ragged last row
+    (144, 512, 513),     # a second token tile
+])
+def test_gemm_tile_edges(ctx, name, rows, cols, tokens):
+    """Edges of the row tiles (16, 128, 256), of N (16 / 32, 256, 512) and of the K-steps, against the rounded operands
+    in f64.  An f32 sum of K products differs from it by at most K * 2^-24 of the sum of their magnitudes."""
+    t = H.TYPES[name]
+    wh = ctx.upload(H.quantized(t, 23, rows, cols), t, rows, cols)
+    w = torch.empty((rows, cols), device="cuda")
+    ctx.dequantize(wh, device_out=w)
+    xb = torch.from_numpy(Q.normal(24, (tokens, cols), 1.0)).cuda().to(torch.bfloat16)
+    y = ctx.gemm_prefill(wh, xb)
+    ctx.synchronize()
+    wb = w.to(torch.bfloat16).double()
+    ref, bound = xb.double() @ wb.T, cols * 2.0 ** -24 * (xb.double().abs() @ wb.abs().T)
+    assert bool(((y.double() - ref).abs() <= bound).all()), float(((y.double() - ref).abs() - bound).max())
+    assert torch.equal(y, ctx.gemm_prefill(wh, xb))
+    wh.free()
