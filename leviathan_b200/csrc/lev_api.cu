@@ -252,6 +252,7 @@ int lev_weights_create(lev_ctx* ctx, const void* bytes, size_t n_bytes, int type
     if (!st) st = lev_launch_scale_check(ctx, w);
     int bits = 0;
     if (!st) st = lev_read_status(ctx, &bits);
+    w->large_scale = (bits & LEV_DEV_LARGE_SCALE) != 0;
     if (!st && (bits & LEV_DEV_NONFINITE_SCALE)) st = lev_fail(ctx, LEV_NONFINITE_SCALE, "a block scale is Inf or NaN");
     if (!st && repack) st = lev_repack_weights(ctx, w);
     if (st) {

@@ -19,6 +19,7 @@
 #define LEV_DEV_NONFINITE_SCALE 2
 #define LEV_DEV_NONFINITE_OUTPUT 4
 #define LEV_DEV_TIMEOUT 8
+#define LEV_DEV_LARGE_SCALE 32  // upload: a block scale whose products leave the f16 range
 #define LEV_DEV_BAD_INDEX 16  // a slot, position or block-table entry outside the cache layout
 
 // Row (in units of rows of head_dim elements) of (block, position inside the block, KV head) in a paged cache pool.
@@ -81,6 +82,7 @@ struct lev_weights {
     size_t packed_bytes;
     int64_t packed_rows;  // rows rounded up to the 16-row tile
     int owns_raw;
+    int large_scale;      // some |d| is 4096 or more: d * (q - 8) may leave the f16 range
 };
 
 struct lev_moe_weights {

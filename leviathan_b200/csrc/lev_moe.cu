@@ -387,6 +387,7 @@ struct GroupArgs {
     int* job_token;      // [max_jobs][cmax] token of each column, -1 = none
     int* job_pos;        // [max_jobs][cmax] grouped position, -1 = none
     int* job_pair;       // [max_jobs][cmax] pair id, -1 = none
+    int4* job_desc;      // [max_jobs] {local expert, first grouped position, columns, 0}, in place of the four tables above
     int* status;
 };
 
@@ -632,6 +633,9 @@ __global__ void __launch_bounds__(1024) k_group(GroupArgs G) {
             }
             seen += __popc(mask);
         }
+        if (G.job_desc)
+            for (int j = lane; j * G.cmax < hist[e]; j += 32)
+                G.job_desc[jobbase[e] + j] = make_int4(e - G.first, offs[e] + j * G.cmax, min(hist[e] - j * G.cmax, G.cmax), 0);
         if (G.job_slice) {
             int nj = (hist[e] + G.cmax - 1) / G.cmax;
             for (int j = lane; j < nj; j += 32) G.job_slice[jobbase[e] + j] = e - G.first;
@@ -721,12 +725,14 @@ __global__ void __launch_bounds__(1024) k_group_fast(GroupArgs G, int nchunks) {
     for (int e = tid; e < G.experts; e += blockDim.x) {
         G.counts[e] = hist[e];
         G.offsets[e] = offs[e];
+        if (G.job_desc && e >= G.first && e < G.first + G.count)
+            for (int j = 0; j * G.cmax < hist[e]; j++)
+                G.job_desc[jobbase[e] + j] = make_int4(e - G.first, offs[e] + j * G.cmax, min(hist[e] - j * G.cmax, G.cmax), 0);
         if (G.job_slice && e >= G.first && e < G.first + G.count) {
             const int nj = (hist[e] + G.cmax - 1) / G.cmax;
             for (int j = 0; j < nj; j++) G.job_slice[jobbase[e] + j] = e - G.first;
-            // empty columns of the expert's last job (wide jobs, which only the grouped GEMM uses, are
-            // described by their first position and the expert's count: their tails are not filled)
-            for (int r = hist[e]; r < nj * G.cmax && G.cmax <= 8; r++) {
+            // empty columns of the expert's last job
+            for (int r = hist[e]; r < nj * G.cmax; r++) {
                 const int q = (jobbase[e] + nj - 1) * G.cmax + (r - (nj - 1) * G.cmax);
                 G.job_token[q] = -1;
                 G.job_pos[q] = -1;
@@ -940,19 +946,17 @@ static int route_dev_impl(lev_ctx* ctx, const lev_moe_weights* w, const float* x
     return lev_cuda_check(ctx, cudaGetLastError(), "k_router_topk");
 }
 
-// grouped dequant-GEMM on the tensor cores (lev_gemm_tc.cu)
-bool lev_gemm_grouped_supported(const lev_weights* w, int rows_per_expert);
-int lev_gemm_grouped_job_tokens(void);
-int lev_gemm_grouped_run(lev_ctx* ctx, const lev_weights* w, int rows_per_expert, const void* xg_bf16, int64_t capacity_rows,
-                         int max_jobs, const int* njobs, const int* job_slice, const int* job_pos, const int* offsets,
-                         int first_expert, const int* out_row, float* out, int64_t out_ld);
-int lev_gather_bf16(lev_ctx* ctx, const float* x, const int* perm, const int* total_pos, int64_t max_pos, int top_k, int cols,
-                    void* out_bf16);
-int lev_act_grouped_bf16(lev_ctx* ctx, const float* gu, const int* total_pos, int64_t max_pos, int inter, void* out_bf16);
+// grouped dequant-GEMM on the tensor cores (lev_moe_gemm.cu)
+bool lev_moe_gemm_supported(const lev_moe_weights* w);
+int lev_moe_gemm_job_tokens(int64_t pairs, int experts);
+size_t lev_moe_gemm_bytes(const lev_moe_weights* w, int64_t pairs);
+int lev_moe_gemm_run(lev_ctx* ctx, const lev_moe_weights* w, const float* x, int64_t pairs, int top_k, const int* perm, const int* total_pos,
+                     const int* njobs, const int4* jobs, int job_tokens, int max_jobs, void* work, float* y, float* act_out);
 
 struct JobTable {
     int cmax, max_jobs;
     int *njobs, *job_slice, *job_token, *job_pos, *job_pair;
+    int4* job_desc;
 };
 
 static int group_dev(lev_ctx* ctx, const int32_t* idx, int64_t tokens, int top_k, int experts, int first, int count,
@@ -973,6 +977,7 @@ static int group_dev(lev_ctx* ctx, const int32_t* idx, int64_t tokens, int top_k
     G.job_token = jt ? jt->job_token : nullptr;
     G.job_pos = jt ? jt->job_pos : nullptr;
     G.job_pair = jt ? jt->job_pair : nullptr;
+    G.job_desc = jt ? jt->job_desc : nullptr;
     G.status = ctx->d_status;
     size_t smem = (size_t)(3 * experts + 2) * sizeof(int);
     const int nchunks = (G.pairs + 31) / 32;
@@ -1022,11 +1027,16 @@ static bool moe_sliced4(lev_ctx* ctx, const lev_moe_weights* w, int64_t pairs, c
 
 // the grouping tables of a call inside the context's scratch (same layout for the same arguments)
 static int group_tables(lev_ctx* ctx, const lev_moe_weights* w, int64_t pairs, int cmax, int max_jobs, int32_t** counts,
-                        int32_t** offsets, int32_t** perm, JobTable* jt) {
-    size_t ints = (size_t)w->experts * 2 + 1 + pairs + 1 + max_jobs + (size_t)3 * max_jobs * cmax + 64;
+                        int32_t** offsets, int32_t** perm, JobTable* jt, bool wide = false) {
+    size_t ints = (size_t)w->experts * 2 + 1 + pairs + 1 + (wide ? 4 : 1 + (size_t)3 * cmax) * max_jobs + 64;
     void* gb;
     LEV_TRY(lev_scratch(ctx, LEV_SCR_MOE_B, ints * sizeof(int), &gb));
     int* p = (int*)gb;
+    *jt = JobTable{};
+    if (wide) {
+        jt->job_desc = (int4*)p;
+        p += (size_t)4 * max_jobs;
+    }
     *counts = p;
     p += w->experts;
     *offsets = p;
@@ -1037,6 +1047,7 @@ static int group_tables(lev_ctx* ctx, const lev_moe_weights* w, int64_t pairs, i
     jt->max_jobs = max_jobs;
     jt->njobs = p;
     p += 1;
+    if (wide) return LEV_OK;
     jt->job_slice = p;
     p += max_jobs;
     jt->job_token = p;
@@ -1050,21 +1061,19 @@ static int group_tables(lev_ctx* ctx, const lev_moe_weights* w, int64_t pairs, i
 static int experts_dev_impl(lev_ctx* ctx, const lev_moe_weights* w, const float* x, int64_t tokens, int top_k,
                             const int32_t* idx, float* y_pairs, float* act_out, bool pre_grouped) {
     const int64_t pairs = tokens * top_k;
-    const int64_t gu_rows_ = 2 * (int64_t)w->inter;
     // decode-sized calls: one job per (token, slot) pair on the one-launch kernel, whose CTAs
     // build their activation tables themselves (no preparation launches, no table memory)
     const bool sliced = moe_sliced(ctx, w, pairs, x);
-    // prefill-sized calls: grouped dequant-GEMM on the tensor cores (bf16 operands, f32 accumulate;
+    // prefill-sized calls: grouped dequant-GEMM on the tensor cores (f16 operands, f32 accumulate;
     // the 2e-2 bar of tensor-core prefill applies to this form)
     // Mid-sized calls (one job per expert and four of its tokens) take the one-launch kernel as far as its tables
     // allow -- 84 tokens of the 128-expert top-8 shape: 180 us at 64 tokens, 222 at 84, where the grouped GEMM costs a
     // flat 300 us up to about 128 tokens -- and from 1024 pairs on the GEMM is preferred wherever it applies.
     const bool sliced4_early = !sliced && pairs < 1024 && moe_sliced4(ctx, w, pairs, x);
     const int64_t min_pairs = 512;
-    const bool tensor = !sliced && !sliced4_early && pairs >= min_pairs && w->hidden % 4 == 0 && lev_gemm_grouped_supported(w->gate_up, (int)gu_rows_) &&
-                        lev_gemm_grouped_supported(w->down, w->hidden);
+    const bool tensor = !sliced && !sliced4_early && pairs >= min_pairs && lev_moe_gemm_supported(w);
     const bool sliced4 = sliced4_early || (!sliced && !tensor && moe_sliced4(ctx, w, pairs, x));
-    const int cmax = sliced ? 1 : tensor ? lev_gemm_grouped_job_tokens() : sliced4 ? 4 : (pairs <= 2 * (int64_t)w->local_count ? 4 : 8), terms = 2;
+    const int cmax = sliced ? 1 : tensor ? lev_moe_gemm_job_tokens(pairs, w->local_count) : sliced4 ? 4 : (pairs <= 2 * (int64_t)w->local_count ? 4 : 8), terms = 2;
     int64_t mj = (int64_t)w->local_count + pairs / cmax;
     if (mj > pairs) mj = pairs;
     const int max_jobs = (int)mj;
@@ -1072,34 +1081,25 @@ static int experts_dev_impl(lev_ctx* ctx, const lev_moe_weights* w, const float*
     // grouping tables
     int32_t *counts, *offsets, *perm;
     JobTable jt;
-    LEV_TRY(group_tables(ctx, w, pairs, cmax, max_jobs, &counts, &offsets, &perm, &jt));
+    LEV_TRY(group_tables(ctx, w, pairs, cmax, max_jobs, &counts, &offsets, &perm, &jt, tensor));
     if (!pre_grouped)
         LEV_TRY(group_dev(ctx, idx, tokens, top_k, w->experts, w->local_first, w->local_count, counts, offsets, perm, &jt));
 
-    // gate_up: columns = tokens of each job, outputs in grouped order [pos][2*inter]
     const int64_t gu_rows = 2 * (int64_t)w->inter;
+    if (tensor) {
+        void* work;
+        LEV_TRY(lev_scratch(ctx, LEV_SCR_MOE_C, lev_moe_gemm_bytes(w, pairs), &work));
+        return lev_moe_gemm_run(ctx, w, x, pairs, top_k, perm, offsets + w->experts, jt.njobs, jt.job_desc, cmax, max_jobs, work, y_pairs, act_out);
+    }
+    // gate_up: columns = tokens of each job, outputs in grouped order [pos][2*inter]
     size_t tb_gu = lev_stream_table_bytes(w->gate_up, cmax, terms, max_jobs, nullptr);
     size_t tb_dn = lev_stream_table_bytes(w->down, cmax, terms, max_jobs, nullptr);
     size_t tb = tb_gu > tb_dn ? tb_gu : tb_dn;
     size_t gu_bytes = ((size_t)pairs * gu_rows * sizeof(float) + 255) & ~(size_t)255;
-    if (tensor) tb = (((size_t)pairs * w->hidden * 2 + 255) & ~(size_t)255) + (((size_t)pairs * w->inter * 2 + 255) & ~(size_t)255);
     void* cb;
     LEV_TRY(lev_scratch(ctx, LEV_SCR_MOE_C, gu_bytes + tb + 256, &cb));
     float* gu = (float*)cb;
     void* tables = (char*)cb + gu_bytes;
-    if (tensor) {
-        void* xg = tables;
-        void* actg = (char*)tables + (((size_t)pairs * w->hidden * 2 + 255) & ~(size_t)255);
-        const int* total_pos = offsets + w->experts;
-        LEV_TRY(lev_gather_bf16(ctx, x, perm, total_pos, pairs, top_k, w->hidden, xg));
-        LEV_TRY(lev_gemm_grouped_run(ctx, w->gate_up, (int)gu_rows, xg, pairs, max_jobs, jt.njobs, jt.job_slice, jt.job_pos, offsets,
-                                     w->local_first, nullptr, gu, gu_rows));
-        LEV_TRY(lev_act_grouped_bf16(ctx, gu, total_pos, pairs, w->inter, actg));
-        LEV_TRY(lev_gemm_grouped_run(ctx, w->down, w->hidden, actg, pairs, max_jobs, jt.njobs, jt.job_slice, jt.job_pos, offsets,
-                                     w->local_first, perm, y_pairs, w->hidden));
-        if (act_out) LEV_TRY(lev_moe_launch_act(ctx, gu, perm, offsets + w->experts, pairs, w->inter, act_out));
-        return LEV_OK;
-    }
     if (sliced || sliced4) {
         LEV_TRY(lev_dense_jobs_run(ctx, w->gate_up, gu_rows, max_jobs, cmax, jt.njobs, jt.job_slice, jt.job_token, jt.job_pos, x,
                                    w->hidden, 0, gu, gu_rows));

@@ -169,6 +169,7 @@ __global__ void k_scale_check(const uint8_t* __restrict__ w, int64_t blocks, int
         if (type == LEV_GGML_Q4_0) {
             const unsigned short* p = (const unsigned short*)(w + b * LEV_Q4_0_BYTES);
             bad = (p[0] & 0x7C00u) == 0x7C00u;
+            if ((p[0] & 0x7FFFu) >= 0x6C00u) atomicOr(status, LEV_DEV_LARGE_SCALE);
         } else if (type == LEV_GGML_Q4_K) {
             const unsigned short* p = (const unsigned short*)(w + b * LEV_Q4_K_BYTES);
             bad = (p[0] & 0x7C00u) == 0x7C00u || (p[1] & 0x7C00u) == 0x7C00u;
