@@ -212,8 +212,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_gemm_pk(const __grid_constant
         // beside the decode warps, and was what bounded the kernel); a wait that ran out is not branched on: what
         // follows stays in bounds. ----
         if (rank == 0) {
-            unsigned elected;
-            asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(elected));
+            const unsigned elected = elect_lane();
             // D f32, A and B bf16, both K-major
             const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((unsigned)(A.n_part >> 3) << 17) | ((unsigned)((128 * CG) >> 4) << 24);
             Ring st(A.stages), ac(A.acc_stages);
@@ -256,31 +255,27 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_gemm_pk(const __grid_constant
             }
         }
     } else {
-        // ---- token tiles ----
-        if (lane == 0) {
-            pdl_wait();
-            Ring st(A.stages);
-            bool ok = true;
-            for (int tile = unit; tile < total && ok; tile += units) {
-                const PkTile T = pk_tile(A, tile);
-                for (int it = 0; it < T.kt && ok; it++) {
-                    ok = pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
-                    if (!ok) break;
-                    unsigned bar = smem_u32(&full[st.s]);
-                    const unsigned dst = smem + (unsigned)st.s * stage_bytes + PK_W_BYTES;
-                    if (rank == 0) mbar_expect(bar, (unsigned)(A.parts * CG) * part_bytes);
-                    if (CG == 2) bar = map_to_rank(bar, 0);
-                    for (int h = 0; h < A.parts; h++)
-                        pk_tma<CG>(dst + (unsigned)h * part_bytes, &xmap, (T.k0 + it) * PK_KS,
-                                   T.t0 + h * A.n_part + (int)rank * (A.n_part / CG), bar);
-                    st.step(1);
-                }
-            }
-            // the tensor core's last releases have arrived before the CTA goes (they may come from the pair's leader)
-            for (int s = 0; s < A.stages && ok; s++) {
-                ok = pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
+        // ---- token tiles (a wait that ran out is not branched on, as above) ----
+        pdl_wait();
+        const unsigned elected = elect_lane();
+        const unsigned full_c = CG == 2 ? map_to_rank(smem_u32(&full[0]), 0) : smem_u32(&full[0]);
+        Ring st(A.stages);
+        for (int tile = unit; tile < total; tile += units) {
+            const PkTile T = pk_tile(A, tile);
+            const int y0 = T.t0 + (int)rank * (A.n_part / CG);
+            for (int it = 0; it < T.kt; it++) {
+                pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
+                const unsigned bar = full_c + 8u * (unsigned)st.s, dst = smem + (unsigned)st.s * stage_bytes + PK_W_BYTES;
+                if (rank == 0) pk_expect(smem_u32(&full[st.s]), (unsigned)(A.parts * CG) * part_bytes, elected);
+                pk_tma<CG>(dst, &xmap, (T.k0 + it) * PK_KS, y0, bar, elected);
+                if (A.parts == 2) pk_tma<CG>(dst + part_bytes, &xmap, (T.k0 + it) * PK_KS, y0 + A.n_part, bar, elected);
                 st.step(1);
             }
+        }
+        // the tensor core's last releases have arrived before the CTA goes (they may come from the pair's leader)
+        for (int s = 0; s < A.stages; s++) {
+            pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
+            st.step(1);
         }
     }
     __syncwarp();

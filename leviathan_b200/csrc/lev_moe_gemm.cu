@@ -30,7 +30,7 @@ constexpr int MG_RAW_SLOTS = 3;
 constexpr int MG_DECODE_WARPS = 16;
 constexpr int MG_MMA_WARP = 20, MG_RAW_WARP = 21, MG_X_WARP = 22;
 constexpr int MG_THREADS = (MG_X_WARP + 1) * 32;
-constexpr int MG_BOX_ROWS = 32;                // tokens of one TMA box
+constexpr int MG_BOX_ROWS = 64;                // tokens of one TMA box
 
 struct MgArgs {
     const unsigned char* packed;
@@ -217,8 +217,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
         }
     } else if (warp == MG_MMA_WARP) {
         // ---- MMA issue (see lev_gemm_pk.cu) ----
-        unsigned elected;
-        asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(elected));
+        const unsigned elected = elect_lane();
         Ring st(A.stages), ac(2);
         int cnt = first < total ? __ldcg(A.jobs + first / A.row_tiles).z : 0;
         for (int tile = first; tile < total; tile += units) {
@@ -266,31 +265,31 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
             e = next;
         }
     } else {
-        // ---- token tiles: boxes of 32 positions, as many as the job needs ----
-        if (lane == 0) {
-            Ring st(A.stages);
-            bool ok = true;
-            int4 job = first < total ? __ldcg(A.jobs + first / A.row_tiles) : make_int4(0, 0, 0, 0);
-            for (int tile = first; tile < total && ok; tile += units) {
-                const int4 next = tile + units < total ? __ldcg(A.jobs + (tile + units) / A.row_tiles) : job;
-                const int boxes = (job.z + MG_BOX_ROWS - 1) / MG_BOX_ROWS;
-                for (int u = 0; u < nu && ok; u++) {
-                    ok = pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
-                    if (!ok) break;
-                    const unsigned bar = smem_u32(&full[st.s]), dst = smem + (unsigned)st.s * stage_bytes + KC * MG_CHUNK_BYTES;
-                    mbar_expect(bar, (unsigned)(boxes * KC) * (MG_BOX_ROWS * 128u));
-                    for (int c = 0; c < KC; c++)
-                        for (int b = 0; b < boxes; b++)
-                            pk_tma<1>(dst + (unsigned)c * x_chunk + (unsigned)b * (MG_BOX_ROWS * 128u), &xmap, (u * KC + c) * 64,
-                                      job.y + b * MG_BOX_ROWS, bar);
-                    st.step(1);
+        // ---- token tiles: boxes of 64 positions, as many as the job needs ----
+        const unsigned elected = elect_lane();
+        Ring st(A.stages);
+        int4 job = first < total ? __ldcg(A.jobs + first / A.row_tiles) : make_int4(0, 0, 0, 0);
+        for (int tile = first; tile < total; tile += units) {
+            const int4 next = tile + units < total ? __ldcg(A.jobs + (tile + units) / A.row_tiles) : job;
+            const int pos0 = __shfl_sync(0xffffffffu, job.y, 0), boxes = (__shfl_sync(0xffffffffu, job.z, 0) + MG_BOX_ROWS - 1) / MG_BOX_ROWS;
+            for (int u = 0; u < nu; u++) {
+                pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
+                const unsigned bar = smem_u32(&full[st.s]), dst = smem + (unsigned)st.s * stage_bytes + KC * MG_CHUNK_BYTES;
+                pk_expect(bar, (unsigned)(boxes * KC) * (MG_BOX_ROWS * 128u), elected);
+                if (KC == 2) {   // jobs of up to 64 tokens
+                    pk_tma<1>(dst, &xmap, u * 128, pos0, bar, elected);
+                    pk_tma<1>(dst + x_chunk, &xmap, u * 128 + 64, pos0, bar, elected);
+                } else {
+                    for (int b = 0; b < boxes; b++)
+                        pk_tma<1>(dst + (unsigned)b * (MG_BOX_ROWS * 128u), &xmap, u * 64, pos0 + b * MG_BOX_ROWS, bar, elected);
                 }
-                job = next;
-            }
-            for (int s = 0; s < A.stages && ok; s++) {   // the tensor core's last releases
-                ok = pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
                 st.step(1);
             }
+            job = next;
+        }
+        for (int s = 0; s < A.stages; s++) {   // the tensor core's last releases
+            pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
+            st.step(1);
         }
     }
     __syncwarp();

@@ -112,18 +112,32 @@ __device__ __forceinline__ void pk_commit(unsigned bar, unsigned elected) {
             "r"(elected)
             : "memory");
 }
-// one box of the token tile; bar is a cluster address (the leader's barrier for a CTA pair)
+// One box of the token tile; bar is a cluster address (the leader's barrier for a CTA pair).  Like the MMAs, issued by
+// the elected lane of a converged warp: from a single-lane branch one box took 250 cycles to issue.
 template <int CG>
-__device__ __forceinline__ void pk_tma(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+__device__ __forceinline__ void pk_tma(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar, unsigned elected) {
     if (CG == 2)
         asm volatile(
-            "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-            "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+            "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+            " @q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n" ::"r"(dst),
+            "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar), "r"(elected)
             : "memory");
     else
-        asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(dst),
-                     "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-                     : "memory");
+        asm volatile(
+            "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+            " @q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n}\n" ::"r"(dst),
+            "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar), "r"(elected)
+            : "memory");
+}
+__device__ __forceinline__ void pk_expect(unsigned bar, unsigned bytes, unsigned elected) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n}\n" ::"r"(bar), "r"(bytes), "r"(elected)
+        : "memory");
+}
+__device__ __forceinline__ unsigned elect_lane() {
+    unsigned e;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+    return e;
 }
 
 __device__ __forceinline__ void tmem_ld32(unsigned a, unsigned* v) {
