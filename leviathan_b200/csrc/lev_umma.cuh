@@ -35,11 +35,21 @@ __device__ __forceinline__ unsigned pk_try(unsigned bar, unsigned parity) {
 }
 // bounded wait; false on timeout or when another thread of the CTA has already given up.  The polls are spaced by
 // the loop's bookkeeping: a tight poll loop takes issue slots from the decode warps.
+// the same with the thread suspended for up to 20 us meanwhile: the polls of idle warps take issue slots otherwise
+__device__ __forceinline__ unsigned pk_try_suspended(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(20000u)
+        : "memory");
+    return ok;
+}
 __device__ __noinline__ bool pk_wait_slow(unsigned bar, unsigned parity, volatile int* abort_flag) {
     long long t_start = 0;
     for (unsigned i = 1;; i++) {
-        if (pk_try(bar, parity)) return true;
-        if ((i & 63u) == 0) {
+        if (pk_try_suspended(bar, parity)) return true;
+        if ((i & 15u) == 0) {
             if (*abort_flag) return false;
             const long long now = clock64();
             if (t_start == 0) t_start = now;
