@@ -27,8 +27,9 @@ namespace {
 constexpr int MG_CHUNK_BYTES = 128 * 64 * 2;   // decoded weights of a 64-column chunk
 constexpr int MG_MAX_STAGES = 6;
 constexpr int MG_RAW_SLOTS = 3;
-constexpr int MG_DECODE_WARPS = 16;
-constexpr int MG_MMA_WARP = 20, MG_RAW_WARP = 21, MG_X_WARP = 22;
+constexpr int MG_TEAMS = 3;                    // teams of eight decode warps, one per 16-row tile
+constexpr int MG_DECODE_WARPS = 8 * MG_TEAMS;
+constexpr int MG_MMA_WARP = MG_DECODE_WARPS + 4, MG_RAW_WARP = MG_MMA_WARP + 1, MG_X_WARP = MG_MMA_WARP + 2;
 constexpr int MG_THREADS = (MG_X_WARP + 1) * 32;
 constexpr int MG_BOX_ROWS = 64;                // tokens of one TMA box
 
@@ -81,6 +82,10 @@ __device__ __forceinline__ void q40_chunk_f16(unsigned raw, int c, unsigned wt, 
     }
 }
 
+__device__ __forceinline__ void mbar_arrive_n(unsigned bar, unsigned n) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(n) : "memory");
+}
+
 // GATE_UP: the expert's gate_up tensor and the fused activation; else the down tensor.  KC: chunks per stage.
 template <bool GATE_UP, int KC>
 __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ MgArgs A) {
@@ -104,7 +109,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
         }
         for (int s = 0; s < MG_RAW_SLOTS; s++) {
             mbar_init(smem_u32(&full_raw[s]), 1);
-            mbar_init(smem_u32(&empty_raw[s]), MG_DECODE_WARPS);
+            mbar_init(smem_u32(&empty_raw[s]), 8 * (4 / KC));
         }
         for (int s = 0; s < 2; s++) {
             mbar_init(smem_u32(&acc_full[s]), 1);
@@ -129,43 +134,45 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
     const int tiles16 = A.rows >> 4;       // 16-row tiles of the gate rows / of the expert
 
     if (warp < MG_DECODE_WARPS) {
-        // ---- decode: 16-row tile w & 7 of the CTA tile, stages (KC 1) or halves of a K-step (KC 2) of parity w >> 3 ----
-        const int tl = warp & 7, p = warp >> 3;
+        // ---- decode: 16-row tile w & 7 of the CTA tile, every third stage from w >> 3 on ----
+        const int tl = warp & 7;
         const DecodeLane L = decode_lane<LEV_GGML_Q4_0>(lane);
         const unsigned o0 = L.g * 128u + (((L.t + 4u * L.odd) ^ L.g) << 4);
         Ring st(A.stages), raw(MG_RAW_SLOTS);
-        st.step(p);
+        int u = warp >> 3;                     // stage inside the tile
+        st.step(u);
         const unsigned wt0 = smem + (unsigned)tl * 2048u, raw0 = raw_ring + (unsigned)tl * kStep;
         bool ok = true;
-        auto unit = [&](unsigned src, int c, bool live) {
-            ok &= pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);   // not branched on here: the warp stays together
-            const unsigned wt = wt0 + (unsigned)st.s * stage_bytes;
-            if (live) {
-                q40_chunk_f16(src, c, wt, L, o0);
-                if (KC == 2) q40_chunk_f16(src, c + 1, wt + MG_CHUNK_BYTES, L, o0);
-            }
-            asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&full[st.s]));
-            st.step(2);
-        };
+        constexpr int UPG = 4 / KC;            // stages of a 256-column K-step
+        int at = 0;                            // K-step (of the tile) the raw ring stands at
         for (int tile = first; tile < total && ok; tile += units) {
             const int rt = tile % A.row_tiles;
             const bool live = (GATE_UP ? rt * 4 + (tl >> 1) : rt * 8 + tl) < tiles16;
-            for (int left = nu - p; left + p > 0; left -= 4 / KC) {
+            for (; u < nu; u += MG_TEAMS) {
+                raw.step(u / UPG - at);
+                at = u / UPG;
                 ok = __all_sync(0xffffffffu, pk_wait(smem_u32(&full_raw[raw.s]), raw.ph, abort_flag) & ok);
                 if (!ok) break;
                 const unsigned src = raw0 + (unsigned)raw.s * (8u * kStep);
-                if (left > 0) unit(src, KC == 2 ? 2 * p : p, live);
-                if (KC == 1 && left > 2) unit(src, p + 2, live);
-                if (lane == 0) mbar_arrive(smem_u32(&empty_raw[raw.s]));
-                raw.step(1);
+                const int c = (u % UPG) * KC;
+                ok &= pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);   // not branched on here: the warp stays together
+                const unsigned wt = wt0 + (unsigned)st.s * stage_bytes;
+                if (live) {
+                    q40_chunk_f16(src, c, wt, L, o0);
+                    if (KC == 2) q40_chunk_f16(src, c + 1, wt + MG_CHUNK_BYTES, L, o0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(smem_u32(&full[st.s]));
+                    // one release per stage of the K-step; the tile's last stage also gives those that do not exist
+                    mbar_arrive_n(smem_u32(&empty_raw[raw.s]), u == nu - 1 ? UPG - u % UPG : 1);
+                }
+                st.step(MG_TEAMS);
             }
             ok = __all_sync(0xffffffffu, ok);
-            if (nu & 1) {   // an odd number of stages: the parities change places
-                if (p) st.step(1);
-                else st.back();
-            }
+            u -= nu;
+            at -= A.spt;
         }
     } else if (warp < MG_MMA_WARP) {
         // ---- epilogue: lane = weight row, columns = tokens ----
@@ -179,31 +186,29 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
             if (!__all_sync(0xffffffffu, pk_wait(smem_u32(&acc_full[ac.s]), ac.ph, abort_flag))) break;
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             const unsigned src = tmem_base + ((unsigned)(quarter * 32) << 16) + (unsigned)ac.s * 256u;
-            const int n16 = (job.z + 15) & ~15;
 #pragma unroll 1
-            for (int c = 0; c < job.z; c += 32) {
-                const int mine = c + lane < job.z ? job.y + c + lane : job.y;   // this lane's column: its position,
-                const float sc = __ldcg(A.scale + mine);                        // scale and output row
+            for (int c = 0; c < job.z; c += 16) {
+                const int mine = c + (lane & 15) < job.z ? job.y + c + (lane & 15) : job.y;   // this lane's column: its position,
+                const float sc = __ldcg(A.scale + mine);                                     // scale and output row
                 const int orow = GATE_UP ? mine : __ldcg(A.out_row + mine);
-                unsigned v[32];
-                if (c + 32 <= n16) tmem_ld32(src + (unsigned)c, v);
-                else tmem_ld16(src + (unsigned)c, v);
+                unsigned v[16];
+                tmem_ld16(src + (unsigned)c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
                 if (GATE_UP) {
                     // lanes 0..15 hold gate rows, 16..31 the up rows that go with them: the lower half takes columns
-                    // c .. c + 15, the upper half c + 16 .. c + 31
+                    // c .. c + 7, the upper half c + 8 .. c + 15
                     const bool up = lane >= 16;
 #pragma unroll
-                    for (int q = 0; q < 16; q++) {
-                        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? v[q] : v[16 + q]), 16);
-                        const float g0 = up ? got : __uint_as_float(v[q]), u0 = up ? __uint_as_float(v[16 + q]) : got;
-                        const int col = q + (up ? 16 : 0);
+                    for (int q = 0; q < 8; q++) {
+                        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(up ? v[q] : v[8 + q]), 16);
+                        const float g0 = up ? got : __uint_as_float(v[q]), u0 = up ? __uint_as_float(v[8 + q]) : got;
+                        const int col = q + (up ? 8 : 0);
                         const float s = __shfl_sync(0xffffffffu, sc, col);
                         if (live && c + col < job.z) A.out[(int64_t)(job.y + c + col) * A.rows + row] = gelu_tanh_up(g0 * s, u0 * s);
                     }
                 } else {
 #pragma unroll
-                    for (int q = 0; q < 32; q++) {
+                    for (int q = 0; q < 16; q++) {
                         const float s = __shfl_sync(0xffffffffu, sc, q);
                         const int o = __shfl_sync(0xffffffffu, orow, q);
                         if (live && c + q < job.z) A.out[(int64_t)o * A.rows + row] = __uint_as_float(v[q]) * s;
