@@ -10,6 +10,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libleviathan_cuda.so")
+HOST_PATH = os.path.join(HERE, "lib", "_pyhost.so")
 
 # status codes (include/leviathan_cuda.h, enum lev_status)
 OK = 0
@@ -152,6 +153,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 def load() -> C.CDLL:
@@ -170,3 +172,21 @@ def load() -> C.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def host():
+    """The native calls of csrc/lev_pyhost.c: the same entry points for the calls made per token, without ctypes'
+    argument conversion.  Raises if it is not built, like load()."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m leviathan_b200.build`")
+        import importlib.machinery
+        import importlib.util
+
+        loader = importlib.machinery.ExtensionFileLoader("_pyhost", HOST_PATH)
+        spec = importlib.util.spec_from_loader("_pyhost", loader)
+        _host = importlib.util.module_from_spec(spec)
+        loader.exec_module(_host)
+    return _host

@@ -15,6 +15,9 @@ import numpy as np
 from . import _lib as L
 
 
+_PROLOGUE = {None: L.PROLOGUE_NONE, "rmsnorm": L.PROLOGUE_RMSNORM, "gelu_up": L.PROLOGUE_GELU_UP}
+
+
 class LevError(RuntimeError):
     """A non-zero lev_status; `.name` is the reference's error-case name."""
 
@@ -37,9 +40,19 @@ def _ptr(a):
     return a.ctypes.data
 
 
+def _raw_stream(device: int) -> int:
+    """torch's current stream of a device as a cudaStream_t value."""
+    global _raw_stream
+    import torch
+
+    f = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # no Stream object is made
+    _raw_stream = f or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+    return _raw_stream(device)
+
+
 class Weights:
     def __init__(self, ctx: "Context", handle, ggml_type: int, rows: int, cols: int, gguf_bytes: int):
-        self.ctx, self.handle = ctx, handle
+        self.ctx, self.handle, self._h = ctx, handle, handle.value
         self.ggml_type, self.rows, self.cols, self.gguf_bytes = ggml_type, rows, cols, gguf_bytes
 
     def release_gguf(self):
@@ -50,12 +63,12 @@ class Weights:
     def free(self):
         if self.handle:
             self.ctx.lib.lev_weights_free(self.ctx.handle, self.handle)
-            self.handle = None
+            self.handle = self._h = None
 
 
 class MoEWeights:
     def __init__(self, ctx: "Context", handle, experts, hidden, inter, local_first, local_count):
-        self.ctx, self.handle = ctx, handle
+        self.ctx, self.handle, self._h = ctx, handle, handle.value
         self.experts, self.hidden, self.inter = experts, hidden, inter
         self.local_first, self.local_count = local_first, local_count
 
@@ -66,7 +79,7 @@ class MoEWeights:
     def free(self):
         if self.handle:
             self.ctx.lib.lev_moe_weights_free(self.ctx.handle, self.handle)
-            self.handle = None
+            self.handle = self._h = None
 
 
 class Context:
@@ -78,12 +91,12 @@ class Context:
         ordering rules hold between this library's kernels and torch's."""
         self.follow_torch_stream = follow_torch_stream
         self._stream_seen = None
-        self.lib = L.load()
+        self.lib, self.host = L.load(), L.host()
         h = C.c_void_p()
         st = self.lib.lev_cuda_init(device, C.byref(h))
         if st != L.OK:
             raise LevError(st, f"lev_cuda_init(device={device})")
-        self.handle = h
+        self.handle, self._h = h, h.value
         self.device = device
 
     # -- plumbing --
@@ -94,7 +107,7 @@ class Context:
     def close(self):
         if self.handle:
             self.lib.lev_cuda_destroy(self.handle)
-            self.handle = None
+            self.handle = self._h = None
 
     def __enter__(self):
         return self
@@ -132,9 +145,7 @@ class Context:
 
     def _flags(self, host: bool, check_finite: bool) -> int:
         if not host and self.follow_torch_stream:
-            import torch
-
-            s = torch.cuda.current_stream(self.device).cuda_stream
+            s = _raw_stream(self.device)
             if s != self._stream_seen:
                 self.set_stream(s)
                 self._stream_seen = s
@@ -144,7 +155,8 @@ class Context:
         if _is_torch(like):
             import torch
 
-            return torch.empty(shape, dtype=getattr(torch, dtype_torch_name), device=like.device)
+            dtype = getattr(torch, dtype_torch_name)
+            return like.new_empty(shape) if like.dtype is dtype else like.new_empty(shape, dtype=dtype)
         return np.empty(shape, dtype_np)
 
     # -- weights --
@@ -191,8 +203,8 @@ class Context:
         if out is None:
             out = self._empty_like_io(x, (n_cols, max(rows, 0)), np.float32, "float32")
         cap = out.size if host else out.numel()
-        self._check(self.lib.lev_matvec(self.handle, w.handle, row0, rows, _ptr(x), x_count, n_cols, _ptr(out), cap,
-                                        schedule, self._flags(host, check_finite)))
+        self._check(self.host.matvec(self._h, w._h, row0, rows, _ptr(x), x_count, n_cols, _ptr(out), cap, schedule,
+                                     self._flags(host, check_finite)))
         return out[0] if one_d else out
 
     def matvec_multi(self, ws, x, outs=None, check_finite: bool = False):
@@ -237,7 +249,7 @@ class Context:
         out = torch.empty_like(x2) if out is None else out
         inv = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device) if want_inverse else None
         self._flags(False, False)
-        self._check(self.lib.lev_rmsnorm(self.handle, _ptr(x2), x2.shape[0], x2.shape[1], _ptr(weight), eps, _ptr(out), _ptr(inv)))
+        self._check(self.host.rmsnorm(self._h, _ptr(x2), x2.shape[0], x2.shape[1], _ptr(weight), eps, _ptr(out), _ptr(inv)))
         out = out.reshape(x.shape)
         return (out, inv) if want_inverse else out
 
@@ -267,7 +279,7 @@ class Context:
 
         out = torch.empty_like(r) if out is None else out
         self._flags(False, False)
-        self._check(self.lib.lev_axpy(self.handle, alpha, _ptr(x), _ptr(r), x.numel(), _ptr(out)))
+        self._check(self.host.axpy(self._h, alpha, _ptr(x), _ptr(r), x.numel(), _ptr(out)))
         return out
 
     def qkv_norm_rope(self, qkv, q_heads: int, kv_heads: int, head_dim: int, q_weight=None, k_weight=None, eps: float = 1e-6,
@@ -331,8 +343,7 @@ class Context:
 
     @staticmethod
     def _fusion(prologue, norm_weight, eps, residual, alpha):
-        code = {None: L.PROLOGUE_NONE, "rmsnorm": L.PROLOGUE_RMSNORM, "gelu_up": L.PROLOGUE_GELU_UP}[prologue]
-        return L.Fusion(code, _ptr(norm_weight), eps, _ptr(residual), alpha)
+        return L.Fusion(_PROLOGUE[prologue], _ptr(norm_weight), eps, _ptr(residual), alpha)
 
     def matvec_fused(self, w: Weights, x, prologue=None, norm_weight=None, eps: float = 1e-6, residual=None,
                      alpha: float = 1.0, row0: int = 0, rows: int | None = None, out=None):
@@ -346,10 +357,9 @@ class Context:
         n_cols = 1 if one_d else x.shape[0]
         if out is None:
             out = torch.empty((n_cols, max(rows, 0)), dtype=torch.float32, device=x.device)
-        f = self._fusion(prologue, norm_weight, eps, residual, alpha)
         self._flags(False, False)
-        self._check(self.lib.lev_matvec_fused(self.handle, w.handle, row0, rows, _ptr(x), x.numel(), n_cols, C.byref(f),
-                                              _ptr(out), out.numel()))
+        self._check(self.host.matvec_fused(self._h, w._h, row0, rows, _ptr(x), x.numel(), n_cols, _PROLOGUE[prologue], _ptr(norm_weight), eps,
+                                           _ptr(residual), alpha, _ptr(out), out.numel()))
         return out[0] if one_d and out.ndim == 2 else out
 
     def matvec_multi_fused(self, ws, x, prologue=None, norm_weight=None, eps: float = 1e-6, outs=None):
@@ -379,10 +389,10 @@ class Context:
 
     def chain_submit(self, prepared):
         """Submits a list built by chain_prepare: the bare C call, for loops that reuse the same buffers."""
-        n, arr, flags, host, _keep = prepared
+        n, arr, flags, host, keep = prepared
         if not host:
             self._flags(False, False)
-        self._check(self.lib.lev_matvec_chain(self.handle, n, arr, flags))
+        self._check(self.host.matvec_chain(self._h, n, keep[0], flags))
 
     def chain_prepare(self, ops, check_finite: bool = False):
         """The lev_chain_op array of a list (see matvec_chain), built once; the buffers it names must stay alive."""
@@ -401,15 +411,15 @@ class Context:
             f = self._fusion(o.get("prologue"), o.get("norm_weight"), o.get("eps", 1e-6), o.get("residual"), o.get("alpha", 1.0))
             arr[i] = L.ChainOp(w.handle, row0, rows, _ptr(x), _ptr(out), int(bool(o.get("depends", False))), f)
         flags = self._flags(host, check_finite)
-        return n, arr, flags, host, [(o["x"], o["out"], o.get("residual"), o.get("norm_weight")) for o in ops]
+        return n, arr, flags, host, (C.addressof(arr), [(o["x"], o["out"], o.get("residual"), o.get("norm_weight")) for o in ops])
 
     # -- decode attention over a paged KV cache (torch CUDA tensors only) --
     def kv_append(self, cache: "PagedKV", slot, pos, k, v):
         """lev_kv_append: k, v f32 [n_cols][kv_heads][head_dim] to position pos[c] of sequence slot[c]."""
         k, v = k.contiguous(), v.contiguous()  # held until the launch is queued
         self._flags(False, False)
-        self._check(self.lib.lev_kv_append(self.handle, C.byref(cache.layout), _ptr(cache.k), _ptr(cache.v), _ptr(cache.table),
-                                           _ptr(slot), _ptr(pos), int(slot.numel()), _ptr(k), _ptr(v)))
+        self._check(self.host.kv_append(self._h, C.addressof(cache.layout), _ptr(cache.k), _ptr(cache.v), _ptr(cache.table), _ptr(slot),
+                                        _ptr(pos), slot.numel(), _ptr(k), _ptr(v)))
 
     def attn_decode(self, cache: "PagedKV", slot, pos, q, window: int = 0, scale: float = 1.0, out=None):
         """lev_attn_decode: q f32 [n_cols][q_heads][head_dim] -> out of the same shape."""
@@ -418,8 +428,9 @@ class Context:
         q = q.contiguous()
         out = torch.empty_like(q) if out is None else out
         self._flags(False, False)
-        self._check(self.lib.lev_attn_decode(self.handle, C.byref(cache.layout), _ptr(cache.k), _ptr(cache.v), _ptr(cache.table),
-                                             _ptr(slot), _ptr(pos), q.shape[0], q.shape[1], _ptr(q), window, scale, _ptr(out)))
+        n_cols, q_heads = q.shape[:2]
+        self._check(self.host.attn_decode(self._h, C.addressof(cache.layout), _ptr(cache.k), _ptr(cache.v), _ptr(cache.table), _ptr(slot),
+                                          _ptr(pos), n_cols, q_heads, _ptr(q), window, scale, _ptr(out)))
         return out
 
     def attn_decode_fused_rows(self, cache: "PagedKV", slot, pos, qkv, q_heads: int, window: int = 0, scale: float = 1.0, out=None):
@@ -462,9 +473,9 @@ class Context:
     def act_bf16(self, x, out=None):
         import torch
 
-        out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device) if out is None else out
+        out = x.new_empty(x.shape, dtype=torch.bfloat16) if out is None else out
         self._flags(False, False)
-        self._check(self.lib.lev_act_bf16(self.handle, _ptr(x.contiguous()), x.numel(), _ptr(out)))
+        self._check(self.host.act_bf16(self._h, _ptr(x.contiguous()), x.numel(), _ptr(out)))
         return out
 
     def gemm_prefill(self, w: Weights, x_bf16, out=None):
@@ -476,7 +487,7 @@ class Context:
         if out is None:
             out = torch.empty((tokens, w.rows), dtype=torch.float32, device=x_bf16.device)
         self._flags(False, False)
-        self._check(self.lib.lev_gemm_prefill(self.handle, w.handle, _ptr(x_bf16), tokens, _ptr(out), 0))
+        self._check(self.host.gemm_prefill(self._h, w._h, _ptr(x_bf16), tokens, _ptr(out), 0))
         return out
 
     # -- MoE --
@@ -551,9 +562,11 @@ class Context:
             out = self._empty_like_io(x, (tokens, mw.hidden), np.float32, "float32")
         idx = self._empty_like_io(x, (tokens, top_k), np.int32, "int32") if want_routing else None
         wts = self._empty_like_io(x, (tokens, top_k), np.float32, "float32") if want_routing else None
-        fn = self.lib.lev_moe_layer_ep if expert_parallel else self.lib.lev_moe_layer
-        self._check(fn(self.handle, mw.handle, _ptr(x), tokens, top_k, _ptr(out), _ptr(idx), _ptr(wts),
-                       self._flags(host, check_finite)))
+        flags = self._flags(host, check_finite)
+        if expert_parallel:
+            self._check(self.lib.lev_moe_layer_ep(self.handle, mw.handle, _ptr(x), tokens, top_k, _ptr(out), _ptr(idx), _ptr(wts), flags))
+        else:
+            self._check(self.host.moe_layer(self._h, mw._h, _ptr(x), tokens, top_k, _ptr(out), _ptr(idx), _ptr(wts), flags))
         return (out, idx, wts) if want_routing else out
 
     def moe_layer_residual(self, mw: MoEWeights, x, top_k: int, residual, alpha: float = 1.0, out=None):
@@ -562,8 +575,7 @@ class Context:
         x, residual = x.contiguous(), residual.contiguous()
         out = residual if out is None else out
         self._flags(False, False)
-        self._check(self.lib.lev_moe_layer_residual(self.handle, mw.handle, _ptr(x), x.shape[0], top_k, _ptr(residual), float(alpha),
-                                                    _ptr(out), 0))
+        self._check(self.host.moe_layer_residual(self._h, mw._h, _ptr(x), x.shape[0], top_k, _ptr(residual), alpha, _ptr(out), 0))
         return out
 
     # -- op spec --

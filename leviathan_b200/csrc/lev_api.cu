@@ -340,8 +340,9 @@ extern "C" int lev_dequantize(lev_ctx* ctx, const lev_weights* w, int64_t row0, 
 static void note_evidence(lev_ctx* ctx, const char* kernel, const lev_weights* w, int64_t rows, int n_cols,
                           int grid, int block) {
     lev_evidence* e = &ctx->ev;
-    snprintf(e->device_name, sizeof e->device_name, "%.127s", ctx->prop.name);
-    snprintf(e->kernel_name, sizeof e->kernel_name, "%.63s", kernel);
+    // one call in front of every product: plain copies, no formatting
+    if (!e->device_name[0]) snprintf(e->device_name, sizeof e->device_name, "%.127s", ctx->prop.name);
+    strncpy(e->kernel_name, kernel, sizeof e->kernel_name - 1);
     e->out_dim = rows;
     e->in_dim = w->cols;
     e->n_cols = n_cols;
