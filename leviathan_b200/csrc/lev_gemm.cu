@@ -15,6 +15,7 @@
 #include <cuda_fp16.h>
 
 #include "lev_internal.h"
+#include "lev_stream_math.cuh"
 
 // tensor-memory form (lev_gemm_pk.cu)
 bool lev_gemm_tc_supported(const lev_weights* w, const void* x_bf16, int64_t tokens);
@@ -152,9 +153,20 @@ __global__ void __launch_bounds__(128) k_gemm_prefill(const uint8_t* __restrict_
             }
 }
 
-__global__ void k_act_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat16* __restrict__ out) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = __float2bfloat16_rn(x[i]);
+// f32 -> bf16, eight elements per thread and step (two 16-byte loads, one 16-byte store) where both sides are 16-byte
+// aligned; the last n % 8 one by one.  One element per thread took 9 us for 512 x 4096 (12 MB), the launch included.
+__global__ void __launch_bounds__(256) k_act_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat16* __restrict__ out, int vec) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int64_t first = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    const int64_t n8 = vec ? n >> 3 : 0;
+    for (int64_t i = first; i < n8; i += step) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(x) + 2 * i), b = __ldg(reinterpret_cast<const float4*>(x) + 2 * i + 1);
+        alignas(16) const __nv_bfloat162 v[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                                     __floats2bfloat162_rn(b.z, b.w)};
+        reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(v);
+    }
+    for (int64_t i = 8 * n8 + first; i < n; i += step) out[i] = __float2bfloat16_rn(x[i]);
 }
 
 }  // namespace
@@ -162,8 +174,9 @@ __global__ void k_act_bf16(const float* __restrict__ x, int64_t n, __nv_bfloat16
 extern "C" int lev_act_bf16(lev_ctx* ctx, const float* x, int64_t n, void* out_bf16) {
     if (!ctx || !x || !out_bf16 || n <= 0) return LEV_BAD_ARGUMENT;
     LEV_CUDA(ctx, cudaSetDevice(ctx->device));
-    int64_t g = (n + 255) / 256, cap = (int64_t)ctx->prop.multiProcessorCount * 16;
-    k_act_bf16<<<(unsigned)(g > cap ? cap : g), 256, 0, ctx->stream>>>(x, n, (__nv_bfloat16*)out_bf16);
+    const int vec = (((uintptr_t)x | (uintptr_t)out_bf16) & 15) == 0;
+    const int64_t items = vec ? (n + 7) / 8 : n, g = (items + 255) / 256, cap = (int64_t)ctx->prop.multiProcessorCount * 8;
+    LEV_CUDA(ctx, launch_pdl(k_act_bf16, dim3((unsigned)(g > cap ? cap : g)), dim3(256), (size_t)0, ctx->stream, x, n, (__nv_bfloat16*)out_bf16, vec));
     ctx->launches++;
     return lev_cuda_check(ctx, cudaGetLastError(), "k_act_bf16");
 }
