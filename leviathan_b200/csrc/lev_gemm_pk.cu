@@ -348,10 +348,11 @@ PkPlan pk_plan(lev_ctx* ctx, int type, int64_t rows, int64_t kt, int64_t tokens,
 
 template <int TYPE, int CG>
 int launch_pk(lev_ctx* ctx, const CUtensorMap& map, const PkArgs& A, int grid, size_t smem) {
-    static size_t configured[16] = {};
-    if (configured[ctx->device & 15] < smem) {
-        LEV_CUDA(ctx, cudaFuncSetAttribute(k_gemm_pk<TYPE, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured[ctx->device & 15] = smem;
+    static bool configured[16] = {};   // the most a launch may ask for, so that two threads' first calls cannot undercut each other
+    if (!configured[ctx->device & 15]) {
+        LEV_CUDA(ctx, cudaFuncSetAttribute(k_gemm_pk<TYPE, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)ctx->prop.sharedMemPerBlockOptin - 1024));
+        configured[ctx->device & 15] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -383,7 +384,15 @@ int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int6
     if (!enc) return lev_fail(ctx, LEV_UNSUPPORTED, "cuTensorMapEncodeTiled is not available");
     const int64_t kt = (w->cols + PK_KS - 1) / PK_KS;
     const bool can_split = ((uintptr_t)y & 15) == 0 && (tokens * w->rows) % 4 == 0;
-    const PkPlan P = pk_plan(ctx, w->type, w->rows, kt, tokens, can_split);
+    PkPlan P = pk_plan(ctx, w->type, w->rows, kt, tokens, can_split);
+    if (P.splits > 1 && (tokens > 128 || w->type == LEV_GGML_Q6_K)) {
+        // A captured call of prompt size keeps to the caller's buffers: partial products would need scratch that cannot
+        // grow inside a capture, and the graph would hold its address.  (Decode batches of the 4-bit formats split there
+        // too: their callers run the step once before they capture it.)
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        LEV_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
+        if (cs != cudaStreamCaptureStatusNone) P = pk_plan(ctx, w->type, w->rows, kt, tokens, false);
+    }
     CUtensorMap map;
     const cuuint64_t gdim[2] = {(cuuint64_t)w->cols, (cuuint64_t)tokens};
     const cuuint64_t gstride[1] = {(cuuint64_t)w->cols * 2};

@@ -84,3 +84,23 @@ def test_gemm_tile_edges(ctx, name, rows, cols, tokens):
     assert bool(((y.double() - ref).abs() <= bound).all()), float(((y.double() - ref).abs() - bound).max())
     assert torch.equal(y, ctx.gemm_prefill(wh, xb))
     wh.free()
+
+
+def test_prompt_call_captured_first(ctx):
+    """A prompt-sized call whose first use is inside a capture: no work buffer may be needed there."""
+    t = H.TYPES["q6_k"]
+    fresh = lev.Context(0)
+    wh = fresh.upload(H.quantized(t, 61, 512, 4096), t, 512, 4096)
+    xb = torch.from_numpy(Q.normal(62, (300, 4096), 1.0)).cuda().to(torch.bfloat16)
+    y = torch.zeros((300, 512), device="cuda")
+    torch.cuda.synchronize()
+    stream, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        fresh.gemm_prefill(wh, xb, out=y)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = fresh.gemm_prefill(wh, xb)   # may split K: another order of the same f32 sums
+    fresh.synchronize()
+    assert float((y - ref).norm() / ref.norm()) < 4096 * 2.0 ** -24
+    wh.free()
+    fresh.close()
