@@ -337,17 +337,20 @@ __global__ void __launch_bounds__(128) k_rows_f16(const float* __restrict__ x, c
         if (128 * i < pieces && tid + 128 * i < pieces) {
             const float v[8] = {a[i].x, a[i].y, a[i].z, a[i].w, b[i].x, b[i].y, b[i].z, b[i].w};
 #pragma unroll
-            for (int j = 0; j < 8; j++) m = max(m, __float_as_uint(v[j]) & 0x7fffffffu);   // magnitudes order like integers
+            for (int j = 0; j < 8; j++) {
+                const unsigned u = __float_as_uint(v[j]) & 0x7fffffffu;   // magnitudes order like integers
+                if (u < 0x7f800000u) m = max(m, u);
+            }
         }
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if ((tid & 31) == 0) wmax[tid >> 5] = m;
     __syncthreads();
     m = max(max(wmax[0], wmax[1]), max(wmax[2], wmax[3]));
-    // exponent of the maximum e: factor 2^(14 - e), its inverse 2^(e - 14); zero rows and rows with an infinity or NaN
-    // as they are.  Both stay in the normal range: e is held to [-111, 127].
+    // exponent of the largest finite magnitude e: factor 2^(14 - e), its inverse 2^(e - 14); infinities and NaN stay what
+    // they are.  Both stay in the normal range: e is held to [-111, 127].
     int e = (int)(m >> 23) - 127;
-    if (m == 0u || m >= 0x7f800000u) e = 14;
+    if (m == 0u) e = 14;
     if (e < -111) e = -111;
     const float f = __uint_as_float((unsigned)(127 + 14 - e) << 23), inv = __uint_as_float((unsigned)(127 - 14 + e) << 23);
     if (tid == 0) scale[pos] = inv;
@@ -379,10 +382,11 @@ __global__ void k_act_by_pair(const float* __restrict__ act, const int* __restri
 
 template <bool GATE_UP, int KC>
 int launch_mg(lev_ctx* ctx, const CUtensorMap& map, const MgArgs& A, int grid, size_t smem) {
-    static size_t configured[16] = {};
-    if (configured[ctx->device & 15] < smem) {
-        LEV_CUDA(ctx, cudaFuncSetAttribute(k_moe_gemm<GATE_UP, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        configured[ctx->device & 15] = smem;
+    static bool configured[16] = {};   // the most a launch may ask for: see lev_gemm_pk.cu
+    if (!configured[ctx->device & 15]) {
+        LEV_CUDA(ctx, cudaFuncSetAttribute(k_moe_gemm<GATE_UP, KC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)ctx->prop.sharedMemPerBlockOptin - 1024));
+        configured[ctx->device & 15] = true;
     }
     LEV_CUDA(ctx, launch_pdl(k_moe_gemm<GATE_UP, KC>, dim3((unsigned)grid), dim3(MG_THREADS), smem, ctx->stream, map, A));
     ctx->launches++;
