@@ -1,5 +1,5 @@
 // Dense decode matvec of the stream schedule in ONE launch: y[n][rows] = W[rows][K] * x[n][K]
-// for n <= 4 activation columns, over the fragment-major repack (see lev_stream.cu for the
+// for n <= 8 activation columns, over the fragment-major repack (see lev_stream.cu for the
 // layout and the arithmetic).
 //
 // What differs from the general stream kernel:
@@ -570,10 +570,11 @@ int launch_dense(lev_ctx* ctx, int grid, size_t smem, const DenseArgs& A) {
 
 template <int TYPE, int CMAX>
 int launch_dense_w(lev_ctx* ctx, int warps, int grid, size_t smem, const DenseArgs& A) {
-    if (warps == 8) return launch_dense<TYPE, CMAX, 8>(ctx, grid, smem, A);
-    if (warps == 12) return launch_dense<TYPE, CMAX, 12>(ctx, grid, smem, A);
-    if (warps == 16) return launch_dense<TYPE, CMAX, 16>(ctx, grid, smem, A);
-    return launch_dense<TYPE, CMAX, 24>(ctx, grid, smem, A);
+    if constexpr (CMAX > 4) {
+        if (warps == 16) return launch_dense<TYPE, CMAX, 16>(ctx, grid, smem, A);
+        if (warps == 12) return launch_dense<TYPE, CMAX, 12>(ctx, grid, smem, A);
+    }
+    return launch_dense<TYPE, CMAX, 8>(ctx, grid, smem, A);
 }
 
 template <int TYPE>
@@ -583,6 +584,10 @@ int launch_dense_c(lev_ctx* ctx, int cmax, int warps, int grid, size_t smem, con
         case 2: return launch_dense_w<TYPE, 2>(ctx, warps, grid, smem, A);
         case 3: return launch_dense_w<TYPE, 3>(ctx, warps, grid, smem, A);
         case 4: return launch_dense_w<TYPE, 4>(ctx, warps, grid, smem, A);
+        case 5: return launch_dense_w<TYPE, 5>(ctx, warps, grid, smem, A);
+        case 6: return launch_dense_w<TYPE, 6>(ctx, warps, grid, smem, A);
+        case 7: return launch_dense_w<TYPE, 7>(ctx, warps, grid, smem, A);
+        case 8: return launch_dense_w<TYPE, 8>(ctx, warps, grid, smem, A);
     }
     return lev_fail(ctx, LEV_BAD_DIMENSIONS, "columns %d", cmax);
 }
@@ -594,14 +599,25 @@ struct DensePlan {
 
 // Shape of a launch, or false when the tables do not fit beside a useful ring.
 bool dense_plan_tiles(lev_ctx* ctx, const lev_weights* w, int64_t tiles, int n_cols, DensePlan* P) {
-    if (n_cols < 1 || n_cols > 4) return false;
+    if (n_cols < 1 || n_cols > 8) return false;
     const size_t step = step_bytes(w->type);
     const size_t tb = lev_stream_table_bytes(w, n_cols, 2, 1, nullptr);
     const int64_t spt = lev_stream_chunks(w) / 4;
     if (tiles < 1 || tiles * spt > 0x7fffffff / 64) return false;
-    const int warps = 8;
+    int warps = 8;
     // half of an SM's shared memory unless one CTA takes the SM
     size_t cap = (size_t)110 * 1024;
+    if (n_cols > 4) {
+        // Five to eight columns: the tables leave no room for a second CTA, so one takes the SM, with as many warps as
+        // keep two K-steps each in flight (16 up to 3900 columns of K at eight columns).  Served from tables in global memory
+        // behind a preparation launch (k_prepare_x, k_stream) the same calls took: [12288 x 4096] Q4_K 21.2 / 23.9 us at
+        // five / eight columns, 17.7 / 19.9 here; [4096 x 2816] Q4_0 at six 16.7, 9.8 here; [16384 x 2048] Q6_K at five
+        // 23.9, 15.2 here; [512 x 1024] Q4_0 at eight 15.3, 5.3 here.  Of 13 shapes from 200 x 320 to 65536 x 2816 none
+        // was slower.
+        cap = 200 * 1024;
+        warps = tb + 16 * 2 * step <= cap ? 16 : tb + 12 * 2 * step <= cap ? 12 : 8;
+        if (tb + 8 * 2 * step > cap) return false;
+    }
     const int sms = ctx->prop.multiProcessorCount;
     const int grid = (int)(tiles < sms ? tiles : sms);
     const int64_t per_cta = ((tiles + grid - 1) / grid) * spt;
@@ -646,7 +662,7 @@ int launch_multi_c(lev_ctx* ctx, int cmax, int grid, size_t smem, const DenseArg
 
 // Several whole tensors of one format and K against the same activations in one launch.
 bool lev_dense_multi_supported(lev_ctx* ctx, int n_ops, const lev_weights* const* w, const float* x, int n_cols) {
-    if (n_ops < 2 || n_ops > 4 || ((uintptr_t)x & 15) != 0) return false;
+    if (n_ops < 2 || n_ops > 4 || n_cols > 4 || ((uintptr_t)x & 15) != 0) return false;
     int64_t tiles = 0;
     for (int i = 0; i < n_ops; i++) {
         if (!w[i] || !w[i]->packed || w[i]->type != w[0]->type || w[i]->cols != w[0]->cols) return false;

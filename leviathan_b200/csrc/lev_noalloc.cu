@@ -85,8 +85,9 @@ extern "C" int lev_matvec_static_scratch(lev_ctx* ctx, const lev_weights* w, int
         e->gpu_us = 0.f;
         e->status = LEV_OK;
     }
-    // the one-launch kernel builds its tables in shared memory and needs no work buffers at all
-    if (lev_dense_supported(ctx, w, row0, rows, x, n_cols)) return lev_dense_run(ctx, w, row0, rows, x, n_cols, y);
+    // the one-launch kernel builds its tables in shared memory and needs no work buffers at all (up to four columns: the
+    // wider calls of this entry point are documented to use the array)
+    if (n_cols <= 4 && lev_dense_supported(ctx, w, row0, rows, x, n_cols)) return lev_dense_run(ctx, w, row0, rows, x, n_cols, y);
 
     const int terms = lev_stream_terms(n_cols);
     lev_stream_job J = {};

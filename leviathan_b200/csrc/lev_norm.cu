@@ -270,7 +270,8 @@ extern "C" int lev_matvec_fused(lev_ctx* ctx, const lev_weights* w, int64_t row0
         const lev_chain_item it = {w, row0, rows, x, y, 0, &d};
         if (lev_chain_preferred(ctx, 1, &it)) return lev_chain_run(ctx, 1, &it);
     }
-    if (lev_dense_supported(ctx, w, row0, rows, x, n_cols)) {
+    const bool aligned = !fusion || ((uintptr_t)fusion->norm_weight & 15) == 0;   // read in 16-byte vectors
+    if (aligned && lev_dense_supported(ctx, w, row0, rows, x, n_cols)) {
         const lev_dense_fusion d = to_dense(fusion);
         return lev_dense_run(ctx, w, row0, rows, x, n_cols, y, fusion ? &d : nullptr);
     }
@@ -324,12 +325,13 @@ extern "C" int lev_matvec_multi_fused(lev_ctx* ctx, int n_ops, const lev_weights
         for (int i = 0; i < n_ops; i++) it[i] = {w[i], 0, w[i]->rows, x, y[i], 0, &d};
         if (lev_chain_preferred(ctx, n_ops, it)) return lev_chain_run(ctx, n_ops, it);
     }
-    if (lev_dense_multi_supported(ctx, n_ops, w, x, n_cols)) {
+    const bool aligned = !fusion || ((uintptr_t)fusion->norm_weight & 15) == 0;
+    if (aligned && lev_dense_multi_supported(ctx, n_ops, w, x, n_cols)) {
         const lev_dense_fusion d = to_dense(fusion);
         return lev_dense_multi_run(ctx, n_ops, w, x, n_cols, y, fusion ? &d : nullptr);
     }
     // one tensor at a time; the prologue runs once when it has to be staged
-    bool all_dense = true;
+    bool all_dense = aligned;
     for (int i = 0; i < n_ops; i++) all_dense = all_dense && lev_dense_supported(ctx, w[i], 0, w[i]->rows, x, n_cols);
     if (all_dense) {
         const lev_dense_fusion d = to_dense(fusion);

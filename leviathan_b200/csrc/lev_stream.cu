@@ -32,7 +32,7 @@
 // others each warp leaves one f32 per (row, column) in a shared-memory record and the CTA adds
 // the records in warp order after a barrier, so the same call always gives the same bits.
 //
-// This file serves the grouped expert FFN, dense calls with 5..8 columns and dense calls whose
+// This file serves the grouped expert FFN and dense calls whose
 // activation tables do not fit shared memory; lev_dense.cu holds the one-launch kernel for the
 // rest.
 #include "lev_stream.h"

@@ -349,3 +349,20 @@ def test_release_of_the_gguf_order_copy(ctx):
         ctx.dequantize(wh)
     assert e.value.name == "unsupported"
     wh.free()
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q4_k", "q6_k"])
+@pytest.mark.parametrize("n_cols,rows,cols", [(5, 16, 256), (6, 250, 2816), (7, 2401, 1024), (8, 33, 4096), (8, 48, 5632), (5, 32, 9472)])
+def test_five_to_eight_columns_in_one_launch(ctx, name, n_cols, rows, cols):
+    """Sizes at the edges of the plan (16, 12 or 8 warps, then the two-launch kernel), against the f64 oracle."""
+    t = H.TYPES[name]
+    w = H.quantized(t, 51, rows, cols)
+    x = Q.normal(52, (n_cols, cols), 1.0)
+    wh = ctx.upload(w, t, rows, cols)
+    buf, view = H.guarded(n_cols * rows)
+    y = ctx.matvec(wh, torch.from_numpy(x).cuda(), out=view.view(n_cols, rows), check_finite=True)
+    ctx.synchronize()
+    assert H.guards_intact(buf, n_cols * rows)
+    for c in range(n_cols):
+        assert O.max_rel_err(y[c].cpu().numpy(), O.matvec_f64(t, w, rows, cols, x[c])) < H.REPORT_TOL
+    wh.free()
