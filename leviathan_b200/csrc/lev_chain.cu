@@ -11,13 +11,14 @@
 //    (lev_chain_split.h).  A warp streams its share through its own ring of shared-memory slots
 //    filled by cp.async.bulk; the fetch side runs ahead across op boundaries, so the HBM stream
 //    does not pause where one tensor ends and the next begins;
-//  * four helper warps build each op's activation tables (fp16 split terms in mma fragment order,
-//    bias sums) one op ahead of the compute warps, apply the fused prologues (RMSNorm, gelu(gate)*up)
+//  * four helper warps build each op's activation tables (digits or fp16 split terms in mma fragment
+//    order, bias sums) one op ahead of the compute warps, apply the fused prologues (RMSNorm, gelu(gate)*up)
 //    and, where an op reads what earlier ops of the launch wrote, wait on a grid-wide arrival
 //    counter first; compute warps that reach an op whose tables are not ready help to build them;
-//  * arithmetic: the fp16-subnormal tensor-core dot of lev_stream_math.cuh with the eight mma
-//    columns used as four sub-block groups x two activation terms, so one accumulator chain spans a
-//    whole K-step and block scales are applied once per K-step by the lane that owns the sub-block;
+//  * arithmetic (lev_chain_math.cuh): the 4-bit formats in integers, activations as four signed bytes per
+//    K-step's power of two; Q6_K as the fp16-subnormal tensor-core dot of lev_stream_math.cuh with the eight
+//    mma columns used as four sub-block groups x two activation terms.  Block scales are applied once per
+//    K-step by the lane that owns the sub-block;
 //  * tiles shared by warps or by blocks are finished by the last to arrive, adding partial sums in
 //    a fixed order: same call, same bits.
 //
@@ -75,7 +76,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // ---------------------------------------------------------------------------
 template <int TYPE>
 __device__ void build_piece(const ChainOp& P, int piece, int lane, unsigned char* tables, float inv, int* status) {
-    constexpr int CMAX = 1, GLT = 2;
+    constexpr int GLT = 2;
     uint4* xs = reinterpret_cast<uint4*>(tables);
     float* sa = reinterpret_cast<float*>(xs + P.chunks * GLT * 8);
     const int items = P.chunks * 4;
@@ -85,6 +86,7 @@ __device__ void build_piece(const ChainOp& P, int piece, int lane, unsigned char
     const int chunk = i2 >> 2, tt = i2 & 3;
     const float* xr = P.x;
     float xv[4][2][2];
+    float4 xq[4];
 #pragma unroll
     for (int m = 0; m < 4; m++) {
         const int el = chunk * 64 + chunk_col<TYPE>(tt, m, 0, 0);
@@ -104,14 +106,18 @@ __device__ void build_piece(const ChainOp& P, int piece, int lane, unsigned char
         }
         const bool in = el < P.cols;
         const float q[4] = {in ? v.x : 0.f, in ? v.y : 0.f, in ? v.z : 0.f, in ? v.w : 0.f};
+        xq[m] = make_float4(q[0], q[1], q[2], q[3]);
 #pragma unroll
         for (int r = 0; r < 2; r++)
 #pragma unroll
             for (int h = 0; h < 2; h++) xv[m][r][h] = q[chunk_col<TYPE>(tt, m, r, h) - chunk_col<TYPE>(tt, m, 0, 0)];
     }
+    if constexpr (TYPE != LEV_GGML_Q6_K) {
+        if (int_tables<TYPE>(xq, chunk, tt, live, xs, reinterpret_cast<unsigned char*>(sa))) atomicOr(status, LEV_DEV_NONFINITE_INPUT);
+        return;
+    }
     unsigned r0[8], r1[8];
     float seen0[4], seen1[4];
-    float plain[2] = {0.f, 0.f};
     bool bad = false;
 #pragma unroll
     for (int m = 0; m < 4; m++) {
@@ -129,7 +135,6 @@ __device__ void build_piece(const ChainOp& P, int piece, int lane, unsigned char
             r1[m * 2 + r] = *reinterpret_cast<const unsigned*>(&p1);
             seen0[m] += f0.x + f0.y;
             seen1[m] += f1.x + f1.y;
-            plain[m >> 1] += xv[m][r][0] + xv[m][r][1];
         }
     }
     if (live) {
@@ -139,41 +144,17 @@ __device__ void build_piece(const ChainOp& P, int piece, int lane, unsigned char
         e0[8] = make_uint4(r1[0], r1[1], r1[2], r1[3]);
         e0[9] = make_uint4(r1[4], r1[5], r1[6], r1[7]);
     }
-    if (TYPE == LEV_GGML_Q4_K) {
 #pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-            float v = plain[hf];
-            v += __shfl_xor_sync(0xffffffffu, v, 1);
-            v += __shfl_xor_sync(0xffffffffu, v, 2);
-            if (live && tt == 0) sa[(chunk * 2 + hf) * CMAX] = v;
-        }
-    } else if (TYPE == LEV_GGML_Q6_K) {
-#pragma unroll
-        for (int m = 0; m < 4; m++) {
-            const float k = (chunk_hi<TYPE>(m) ? 16.0f : 1.0f) * -32.0f * 5.9604644775390625e-08f;
-            float v0 = seen0[m], v1 = seen1[m];
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
-            if (live && tt == 0) {
-                sa[(chunk * 4 + m) * GLT] = k * v0;
-                sa[(chunk * 4 + m) * GLT + 1] = k * v1;
-            }
-        }
-    } else {
-#pragma unroll
-        for (int blk = 0; blk < 2; blk++) {
-            const float k = -8.0f * 5.9604644775390625e-08f;
-            float v0 = seen0[2 * blk] + 16.0f * seen0[2 * blk + 1], v1 = seen1[2 * blk] + 16.0f * seen1[2 * blk + 1];
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
-            v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
-            v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
-            if (live && tt == 0) {
-                sa[(chunk * 2 + blk) * GLT] = k * v0;
-                sa[(chunk * 2 + blk) * GLT + 1] = k * v1;
-            }
+    for (int m = 0; m < 4; m++) {
+        const float k = (chunk_hi<TYPE>(m) ? 16.0f : 1.0f) * -32.0f * 5.9604644775390625e-08f;
+        float v0 = seen0[m], v1 = seen1[m];
+        v0 += __shfl_xor_sync(0xffffffffu, v0, 1);
+        v1 += __shfl_xor_sync(0xffffffffu, v1, 1);
+        v0 += __shfl_xor_sync(0xffffffffu, v0, 2);
+        v1 += __shfl_xor_sync(0xffffffffu, v1, 2);
+        if (live && tt == 0) {
+            sa[(chunk * 4 + m) * GLT] = k * v0;
+            sa[(chunk * 4 + m) * GLT + 1] = k * v1;
         }
     }
     if (bad) atomicOr(status, LEV_DEV_NONFINITE_INPUT);
@@ -208,7 +189,7 @@ template <int W>
 __global__ void __launch_bounds__((W + kHelperWarps) * 32, 1) k_chain(const __grid_constant__ ChainArgs A) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[W][kRingBars];
-    __shared__ __align__(16) uint4 zero_block[2];
+    __shared__ __align__(16) uint4 zero_block[kZeroBytes / 16];
     __shared__ __align__(16) TileEntry fq[kQueue];
     __shared__ unsigned fq_tail;
     __shared__ volatile unsigned fq_head;
@@ -235,7 +216,7 @@ __global__ void __launch_bounds__((W + kHelperWarps) * 32, 1) k_chain(const __gr
     }
     if (threadIdx.x < W) prog[threadIdx.x] = 0;
     for (int i = threadIdx.x; i < kRecDepth * 2 * W; i += blockDim.x) (&tick[0][0])[i] = 0;
-    if (threadIdx.x < 2) zero_block[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < kZeroBytes / 16) zero_block[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < kQueue) fq[threadIdx.x].ready = 0u;
     if (threadIdx.x == 0) {
         abort_flag = 0;
@@ -388,14 +369,7 @@ __global__ void __launch_bounds__((W + kHelperWarps) * 32, 1) k_chain(const __gr
         // ===================== compute warps =====================
         bool dead = false;
         LaneConst L;
-        L.q_off = 16u * lane;
-        L.hdr_off = 16u * g;
-        L.x_off = (unsigned)(((g & 1) * 4 + t) * 32);
-        L.grp = (unsigned)(g >> 1);
-        L.t = (unsigned)t;
-        L.g = (unsigned)g;
-        L.sh16 = 16u * (t & 1);
-        L.zero_s = smem_u32(zero_block);
+        L.init(lane, smem_u32(zero_block));
         const unsigned smem_s = smem_u32(smem);
         while (c_op < n_ops && !dead) {
             // ---------- enter op ----------
@@ -448,7 +422,7 @@ __global__ void __launch_bounds__((W + kHelperWarps) * 32, 1) k_chain(const __gr
             auto run = [&](auto tag) {
                 constexpr int TYPE = decltype(tag)::value;
                 constexpr u32 bytes = (u32)step_bytes(TYPE), grp = copy_steps(TYPE);
-                constexpr u32 aux_bytes = TYPE == LEV_GGML_Q4_K ? 32u : (TYPE == LEV_GGML_Q6_K ? 128u : 64u);
+                constexpr u32 aux_bytes = kOneColAux<TYPE>;
                 u32 tile = first_tile;
                 u32 k = s - tile * spt, seg_k0 = k;
                 unsigned xk = xs_s + k * 1024u, ak = sa_s + k * aux_bytes;
@@ -473,7 +447,8 @@ __global__ void __launch_bounds__((W + kHelperWarps) * 32, 1) k_chain(const __gr
 #pragma unroll 1
                     for (u32 j = 0; j < grp_n; j++) {
                         {
-                            chain_step<TYPE>(st, xk, ak, L, ya, yb);
+                            if constexpr (TYPE == LEV_GGML_Q6_K) chain_step<TYPE>(st, xk, ak, L, ya, yb);
+                            else int_step<TYPE>(st, xk, ak, L, ya, yb);
                             if (j + 1 == grp_n) {
                                 // every lane has read the copy's bytes: hand them back to the fetch side
                                 __syncwarp();
@@ -795,7 +770,7 @@ static bool chain_plan(lev_ctx* ctx, int n_ops, const lev_chain_item* items, Cha
             slot_owner[slot] = o;
             last_reader[slot] = o;
             last_builder = o;
-            const size_t tb = (lev_stream_table_bytes(w, 1, 2, 1, nullptr) + 255) & ~(size_t)255;
+            const size_t tb = (lev_one_column_table_bytes(w) + 255) & ~(size_t)255;
             if (tb > tab_bytes[slot]) tab_bytes[slot] = tb;
         }
     }
@@ -805,7 +780,7 @@ static bool chain_plan(lev_ctx* ctx, int n_ops, const lev_chain_item* items, Cha
         later_wait |= A->op[o].wait;
     }
     const size_t cap = ctx->prop.sharedMemPerBlockOptin;
-    const size_t fixed_static = 8 * 1024;  // static shared memory of the kernel, rounded up
+    const size_t fixed_static = 9 * 1024;  // static shared memory of the kernel (8320 bytes with 16 warps), rounded up
     // compute warps: with the four helper warps a multiple of four, so that the register file splits evenly
     int warps = ctx->chain_warps == 12 ? 12 : 16;
     for (;; warps = 12) {

@@ -372,14 +372,7 @@ __global__ void __launch_bounds__(W * 32, W <= 8 ? 2 : 1) k_dense(DenseArgs A) {
     // sums of rows g and g + 8, the table layout is the same.
     float ya = 0.f, yb = 0.f;
     LaneConst LC;
-    LC.q_off = 16u * lane;
-    LC.hdr_off = 16u * g;
-    LC.x_off = (unsigned)(((g & 1) * 4 + t) * 32);
-    LC.grp = (unsigned)(g >> 1);
-    LC.t = (unsigned)t;
-    LC.g = (unsigned)g;
-    LC.sh16 = 16u * (t & 1);
-    LC.zero_s = smem_u32(zero_block);
+    LC.init(lane, smem_u32(zero_block));
     unsigned xs_s = 0, sa_s = 0;  // shared-memory addresses of the tables of the tile being worked on
     float yacc[NT][4];
     float mina[CMAX], minb[CMAX];

@@ -36,6 +36,7 @@
 // activation tables do not fit shared memory; lev_dense.cu holds the one-launch kernel for the
 // rest.
 #include "lev_stream.h"
+#include "lev_chain_math.cuh"
 #include "lev_stream_math.cuh"
 
 namespace {
@@ -645,6 +646,12 @@ size_t lev_stream_table_bytes(const lev_weights* w, int cmax, int terms, int job
     ab = (ab + 255) & ~(size_t)255;
     if (frag_bytes) *frag_bytes = fb;
     return fb + ab;
+}
+
+// tables of one column in the arithmetic of lev_chain_math.cuh
+size_t lev_one_column_table_bytes(const lev_weights* w) {
+    const size_t aux = w->type == LEV_GGML_Q4_K ? kOneColAux<LEV_GGML_Q4_K> : w->type == LEV_GGML_Q6_K ? kOneColAux<LEV_GGML_Q6_K> : kOneColAux<LEV_GGML_Q4_0>;
+    return (size_t)(lev_stream_chunks(w) / 4) * (1024 + aux);
 }
 
 static PrepArgs make_prep(lev_ctx* ctx, const lev_weights* w, const lev_stream_source& src, int cmax, int terms,

@@ -28,6 +28,7 @@ struct lev_stream_job {
 int lev_stream_terms(int n_cols);
 int64_t lev_stream_chunks(const lev_weights* w);
 size_t lev_stream_table_bytes(const lev_weights* w, int cmax, int terms, int jobs, size_t* frag_bytes);
+size_t lev_one_column_table_bytes(const lev_weights* w);
 int lev_stream_prepare(lev_ctx* ctx, const lev_weights* w, const lev_stream_source& src, int cmax, int terms, int jobs,
                        void* tables);
 // tables: what lev_stream_prepare wrote for the same (weights, cmax, terms, jobs)

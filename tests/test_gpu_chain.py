@@ -202,3 +202,47 @@ def test_chain_rejections(ctx):
         ctx.matvec_chain([dict(w=wh, x=x, out=y)] * 33)
     assert e.value.name == "badArgument"
     wh.free()
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q4_k"])
+@pytest.mark.parametrize("rows,cols", [(16, 256), (35, 1280), (4096, 2816)])
+@pytest.mark.parametrize("kind", ["normal", "outlier", "tiny", "large", "zero_steps"])
+def test_integer_activations(ctx, name, rows, cols, kind):
+    """The 4-bit formats' integer form over activation ranges: an activation is held to half of 2^-30 of the power of two
+    above its 256 columns' largest (2^-30 of that largest), the sums of a K-step are exact up to the rounding of its few
+    scaled terms, and f32 rounds once per K-step and reduction stage.  A Q4_K term d * sc * q and its min dmin * m are
+    each at most twice the sub-block's largest weight."""
+    t = H.TYPES[name]
+    x = Q.normal(41, (cols,), 1.0)
+    if kind == "outlier":
+        x[cols // 2] = 3.0e4
+    elif kind == "tiny":
+        x *= np.float32(1e-30)
+    elif kind == "large":
+        x *= np.float32(1e9)   # beyond the f16 range
+    elif kind == "zero_steps":
+        x[:256] = 0.0
+    w = H.quantized(t, 42, rows, cols)
+    wh = ctx.upload(w, t, rows, cols)
+    out = ctx.matvec_chain([dict(w=wh, x=_dev(x), out=torch.empty(rows, device="cuda"))])[0]
+    ctx.synchronize()
+    x64 = x.astype(np.float64)
+    deq = O.dequantize_rows(t, w, rows, cols).astype(np.float64)
+    step = np.abs(x64).reshape(-1, 256).max(1).repeat(256) if cols % 256 == 0 else np.abs(x64).max()
+    most = 4.0 * np.abs(deq).max(1)
+    bound = most * ((2.0 ** -30 * step * np.ones(cols)).sum() + (24 + cols / 256) * 2.0 ** -24 * np.abs(x64).sum())
+    err = np.abs(out.cpu().numpy().astype(np.float64) - deq @ x64)
+    assert (err <= bound + 1e-37).all(), float((err - bound).max())
+    wh.free()
+
+
+@pytest.mark.parametrize("name", ["q4_0", "q4_k"])
+def test_integer_activations_not_finite(ctx, name):
+    t = H.TYPES[name]
+    for bad in (np.inf, -np.inf, np.nan):
+        x = Q.normal(43, (512,), 1.0)
+        x[300] = bad
+        wh = ctx.upload(H.quantized(t, 44, 40, 512), t, 40, 512)
+        out = ctx.matvec_chain([dict(w=wh, x=_dev(x), out=torch.empty(40, device="cuda"))])[0]
+        assert not bool(torch.isfinite(out).any())
+        wh.free()
