@@ -73,9 +73,9 @@ __device__ __forceinline__ float byte_to_float_16th(unsigned w, unsigned k) {
 // products and fragment loads are issued, the sums are exact integers, and n keeps an activation to 2^-31 of its K-step's
 // largest (the f16 form's two terms: 2^-22 of its own size, and nothing beyond the f16 range): error against f64 on normal
 // activations 1e-7 (Q4_0) and 2e-7 (Q4_K) of the result where the f16 form shows 9e-7.  FFN set of the persistent kernel
-// 32.3 -> 30.2 us, [12288 x 6144] Q4_K 14.7 -> 13.4 us.  lev_dense.cu stays with the f16 form: job lists of one column lost
-// (27.7 -> 28.2 us for a MoE layer of one token, the tables cost more to build than a short share wins back), and plain
-// products agree with their wider calls there.
+// 32.3 -> 30.2 us, [12288 x 6144] Q4_K 14.7 -> 13.4 us.  lev_dense.cu stays with the f16 form: job lists of one column gained
+// nothing (28.2 against 27.7 us for a MoE layer of one token, where two processes of one build differ by 1.5 %: the tables
+// cost what a short share wins back), and plain products agree with their wider calls there.
 // Table of a K-step: fragments [chunk][digit][quad lane][four mma registers] (1 KB), then kIntAux bytes of sums:
 // Q4_K: activation sums of the eight sub-blocks (f32), Q4_0: -8 * (digit sum) [chunk][digit / 2][block][digit & 1] (s32);
 // then the power of two (f32; NaN where an activation is not finite, so that the results are).
