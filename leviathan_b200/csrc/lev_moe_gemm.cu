@@ -25,9 +25,14 @@
 namespace {
 
 constexpr int MG_CHUNK_BYTES = 128 * 64 * 2;   // decoded weights of a 64-column chunk
-constexpr int MG_MAX_STAGES = 6;
 constexpr int MG_RAW_SLOTS = 3;
 constexpr int MG_TEAMS = 3;                    // teams of eight decode warps, one per 16-row tile
+constexpr int MG_STAGES = 3;                   // 48 KB each in both forms (KC = 1: 256 tokens, KC = 2: 64)
+// A team steps MG_TEAMS stages at a time and may pass over a K-step of the raw ring (a tile whose number of stages is odd
+// ends in a K-step of one stage), where a wait by parity alone could be satisfied by the phase before.  With as many
+// stages as teams the release of a stage says that all stages before it have been decoded: see the decode loop.
+static_assert(MG_STAGES == MG_TEAMS && MG_RAW_SLOTS == 3, "the decode loop's waits rely on it");
+static_assert(MG_STAGES * (MG_CHUNK_BYTES + 256 * 128) + MG_RAW_SLOTS * 8 * (int)kStepBytesQ4 + 1024 <= 225 * 1024, "shared memory of a CTA");
 constexpr int MG_DECODE_WARPS = 8 * MG_TEAMS;
 constexpr int MG_MMA_WARP = MG_DECODE_WARPS + 4, MG_RAW_WARP = MG_MMA_WARP + 1, MG_X_WARP = MG_MMA_WARP + 2;
 constexpr int MG_THREADS = (MG_X_WARP + 1) * 32;
@@ -43,7 +48,7 @@ struct MgArgs {
     const float* scale;     // [position] power of two the activations were divided by
     const int* out_row;     // down: [position] row of out
     float* out;             // gate_up: [position][inter] gelu(gate) * up; down: [out_row][hidden]
-    int job_tokens, stages;
+    int job_tokens;
     int* status;
 };
 
@@ -90,7 +95,7 @@ __device__ __forceinline__ void mbar_arrive_n(unsigned bar, unsigned n) {
 template <bool GATE_UP, int KC>
 __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ MgArgs A) {
     extern __shared__ unsigned char smem_dyn[];
-    __shared__ __align__(8) unsigned long long full[MG_MAX_STAGES], empty[MG_MAX_STAGES];
+    __shared__ __align__(8) unsigned long long full[MG_STAGES], empty[MG_STAGES];
     __shared__ __align__(8) unsigned long long full_raw[MG_RAW_SLOTS], empty_raw[MG_RAW_SLOTS], acc_full[2], acc_empty[2];
     __shared__ unsigned tmem_base_s;
     __shared__ int abort_s;
@@ -99,11 +104,11 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
     const unsigned smem = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     const unsigned x_chunk = (unsigned)A.job_tokens * 128u;             // tokens of one chunk
     const unsigned stage_bytes = KC * (MG_CHUNK_BYTES + x_chunk);       // [KC] weights, [KC] tokens
-    const unsigned raw_ring = smem + (unsigned)A.stages * stage_bytes;
+    const unsigned raw_ring = smem + MG_STAGES * stage_bytes;
 
     if (threadIdx.x == 0) {
         abort_s = 0;
-        for (int s = 0; s < MG_MAX_STAGES; s++) {
+        for (int s = 0; s < MG_STAGES; s++) {
             mbar_init(smem_u32(&full[s]), 1 + 8);
             mbar_init(smem_u32(&empty[s]), 1);
         }
@@ -138,7 +143,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
         const int tl = warp & 7;
         const DecodeLane L = decode_lane<LEV_GGML_Q4_0>(lane);
         const unsigned o0 = L.g * 128u + (((L.t + 4u * L.odd) ^ L.g) << 4);
-        Ring st(A.stages), raw(MG_RAW_SLOTS);
+        Ring st(MG_STAGES), raw(MG_RAW_SLOTS);
         int u = warp >> 3;                     // stage inside the tile
         st.step(u);
         const unsigned wt0 = smem + (unsigned)tl * 2048u, raw0 = raw_ring + (unsigned)tl * kStep;
@@ -151,11 +156,13 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
             for (; u < nu; u += MG_TEAMS) {
                 raw.step(u / UPG - at);
                 at = u / UPG;
+                // The stage first: its release means that every stage up to the one MG_STAGES before has been decoded, so
+                // the K-step that held this raw slot before has landed, and the parity below can only mean this one.
+                ok &= pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
                 ok = __all_sync(0xffffffffu, pk_wait(smem_u32(&full_raw[raw.s]), raw.ph, abort_flag) & ok);
                 if (!ok) break;
                 const unsigned src = raw0 + (unsigned)raw.s * (8u * kStep);
                 const int c = (u % UPG) * KC;
-                ok &= pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);   // not branched on here: the warp stays together
                 const unsigned wt = wt0 + (unsigned)st.s * stage_bytes;
                 if (live) {
                     q40_chunk_f16(src, c, wt, L, o0);
@@ -223,7 +230,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
     } else if (warp == MG_MMA_WARP) {
         // ---- MMA issue (see lev_gemm_pk.cu) ----
         const unsigned elected = elect_lane();
-        Ring st(A.stages), ac(2);
+        Ring st(MG_STAGES), ac(2);
         int cnt = first < total ? __ldcg(A.jobs + first / A.row_tiles).z : 0;
         for (int tile = first; tile < total; tile += units) {
             const int next = tile + units < total ? __ldcg(A.jobs + (tile + units) / A.row_tiles).z : 0;   // a tile ahead
@@ -272,7 +279,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
     } else {
         // ---- token tiles: boxes of 64 positions, as many as the job needs ----
         const unsigned elected = elect_lane();
-        Ring st(A.stages);
+        Ring st(MG_STAGES);
         int4 job = first < total ? __ldcg(A.jobs + first / A.row_tiles) : make_int4(0, 0, 0, 0);
         for (int tile = first; tile < total; tile += units) {
             const int4 next = tile + units < total ? __ldcg(A.jobs + (tile + units) / A.row_tiles) : job;
@@ -292,7 +299,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
             }
             job = next;
         }
-        for (int s = 0; s < A.stages; s++) {   // the tensor core's last releases
+        for (int s = 0; s < MG_STAGES; s++) {   // the tensor core's last releases
             pk_wait(smem_u32(&empty[st.s]), st.ph ^ 1u, abort_flag);
             st.step(1);
         }
@@ -458,10 +465,7 @@ int lev_moe_gemm_run(lev_ctx* ctx, const lev_moe_weights* w, const float* x, int
         A.job_tokens = job_tokens;
         A.status = ctx->d_status;
         const size_t stage = (size_t)kc * (MG_CHUNK_BYTES + job_tokens * 128), raw = (size_t)MG_RAW_SLOTS * 8 * kStepBytesQ4;
-        const size_t cap = ctx->prop.sharedMemPerBlockOptin - 2048;
-        const int64_t fit = (int64_t)((cap - raw) / stage);
-        A.stages = (int)(fit > MG_MAX_STAGES ? MG_MAX_STAGES : fit);
-        const size_t smem = A.stages * stage + raw + 1024;
+        const size_t smem = MG_STAGES * stage + raw + 1024;
         const int64_t most = (int64_t)max_jobs * A.row_tiles;
         const int grid = (int)(most < sms ? most : sms);
         LEV_TRY(half ? (kc == 2 ? launch_mg<false, 2>(ctx, map, A, grid, smem) : launch_mg<false, 1>(ctx, map, A, grid, smem))

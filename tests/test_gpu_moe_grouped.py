@@ -1,0 +1,95 @@
+"""The grouped dequant-GEMM of prefill-sized MoE calls (k_moe_gemm) at the edges of its tiles, stages and jobs, every
+pair against the experts in f64."""
+import numpy as np
+import pytest
+import torch
+
+import leviathan_b200 as lev
+from leviathan_b200 import quant as Q
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = lev.Context(0)
+    yield c
+    c.close()
+
+
+class Layer:
+    def __init__(self, ctx, experts, hidden, inter, seed, edit=None):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        self.dims = experts, hidden, inter
+        self.gu = Q.quantize_q4_0(torch.randn((experts * 2 * inter, hidden), generator=g, device="cuda") * 0.02).cpu().numpy()
+        self.dn = Q.quantize_q4_0(torch.randn((experts * hidden, inter), generator=g, device="cuda") * 0.02).cpu().numpy()
+        if edit:
+            edit(self.gu, self.dn)
+        self.rw = np.zeros((experts, hidden), np.float32)
+        self.mw = ctx.moe_upload(self.rw, self.gu, self.dn, experts, hidden, inter)
+
+    def weights(self):
+        e, h, i = self.dims
+        f64 = lambda b, r, c: torch.from_numpy(O.dequantize_rows(Q.GGML_Q4_0, b, r, c)).cuda().double()
+        return f64(self.gu, e * 2 * i, h).view(e, 2 * i, h), f64(self.dn, e * h, i).view(e, h, i)
+
+
+def reference(layer, x, idx):
+    """(y, bound of y, act, bound of act) per pair in f64.  Operands are rounded once to 11 bits (half a unit: 2^-11 of the
+    value; activations at least 2^-39 of their row's largest), products are exact and K of them are added in f32.  |gelu'|
+    is at most 1.13."""
+    gu, dn = layer.weights()
+    e, h, i = layer.dims
+    t, k = idx.shape
+    x64, flat = x.double(), idx.reshape(-1).long()
+    act = torch.zeros((t * k, i), dtype=torch.float64, device="cuda")
+    act_b, y, y_b = torch.zeros_like(act), torch.zeros((t * k, h), dtype=torch.float64, device="cuda"), None
+    y_b = torch.zeros_like(y)
+
+    def dot(v, v_err, w):
+        rel = 2.0 ** -10 + 2.0 ** -21 + v.shape[1] * 2.0 ** -24
+        lost = 2.0 ** -38 * v.abs().amax(1, keepdim=True) * w.abs().sum(1)
+        return v @ w.T, rel * ((v.abs() + v_err) @ w.abs().T) + v_err @ w.abs().T + lost
+
+    for ex in range(e):
+        p = (flat == ex).nonzero()[:, 0]
+        if not len(p):
+            continue
+        v = x64[p // k]
+        g, g_e = dot(v, torch.zeros_like(v), gu[ex, :i])
+        u, u_e = dot(v, torch.zeros_like(v), gu[ex, i:])
+        gl = torch.nn.functional.gelu(g, approximate="tanh")
+        act[p] = gl * u
+        act_b[p] = 1.13 * g_e * (u.abs() + u_e) + gl.abs() * u_e + 2.0 ** -20 * (gl * u).abs() + 1e-37
+        y[p], y_b[p] = dot(act[p], act_b[p], dn[ex])
+    return y.view(t, k, h), y_b.view(t, k, h), act.view(t, k, i), act_b.view(t, k, i)
+
+
+def routing(rng, tokens, top_k, experts, crowd=0):
+    """top_k different experts per token; the first `crowd` tokens all have expert 1."""
+    idx = np.stack([rng.permutation(experts)[:top_k] for _ in range(tokens)]).astype(np.int32)
+    for t in range(crowd):
+        if 1 not in idx[t]:
+            idx[t, t % top_k] = 1
+    return torch.from_numpy(idx).cuda()
+
+
+def check(ctx, layer, x, idx, times=1):
+    want, bound, _, _ = reference(layer, x, idx)
+    ctx.moe_experts(layer.mw, x, idx)
+    for _ in range(times):
+        y = ctx.moe_experts(layer.mw, x, idx)
+        ctx.synchronize()
+        assert bool(((y.double() - want).abs() <= bound).all()), float(((y.double() - want).abs() / bound).max())
+
+
+@pytest.mark.parametrize("hidden,inter", [(1152, 320), (1408, 384), (2176, 640), (640, 896), (384, 128), (896, 96)])
+def test_odd_numbers_of_stages(ctx, hidden, inter):
+    """Two chunks of 64 columns make a stage of the 64-token jobs: with an odd number of stages a tile ends in a K-step of
+    one stage, and a decode team passes over K-steps of the raw ring."""
+    rng = np.random.default_rng(hidden)
+    layer = Layer(ctx, 32, hidden, inter, hidden + inter)
+    x = torch.from_numpy(Q.normal(hidden, (260, hidden), 1.0)).cuda()
+    check(ctx, layer, x, routing(rng, 260, 4, 32), times=8)
+    layer.mw.free()
