@@ -317,7 +317,9 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
 
 // Activation rows for k_moe_gemm: f32 row (of the token of pair perm[pos], or row pos itself) -> f16, scaled by the
 // power of two that brings its largest magnitude into [2^14, 2^15), 64-column chunks in the column order of
-// q40_word_f16.  One block of 128 threads per position; a thread makes 16-byte pieces from two 16-byte loads.
+// q40_word_f16.  One block of 128 threads per position; a thread makes 16-byte pieces from two 16-byte loads, or from
+// eight single ones where the caller's rows do not start on 16 bytes.
+template <bool VEC>
 __global__ void __launch_bounds__(128) k_rows_f16(const float* __restrict__ x, const int* __restrict__ perm, const int* __restrict__ total_pos,
                                                   int top_k, int cols, uint4* __restrict__ out, float* __restrict__ scale) {
     pdl_launch_dependents();
@@ -334,9 +336,14 @@ __global__ void __launch_bounds__(128) k_rows_f16(const float* __restrict__ x, c
     for (int i = 0; i < kMost; i++) {
         const int d = tid + 128 * i;
         if (128 * i < pieces && d < pieces) {
-            const float4* src = reinterpret_cast<const float4*>(row + (d >> 3) * 64 + ((d >> 2) & 1) * 32 + (d & 3) * 4);
-            a[i] = __ldcg(src);
-            b[i] = __ldcg(src + 4);
+            const float* src = row + (d >> 3) * 64 + ((d >> 2) & 1) * 32 + (d & 3) * 4;
+            if (VEC) {
+                a[i] = __ldcg(reinterpret_cast<const float4*>(src));
+                b[i] = __ldcg(reinterpret_cast<const float4*>(src) + 4);
+            } else {
+                a[i] = make_float4(__ldcg(src), __ldcg(src + 1), __ldcg(src + 2), __ldcg(src + 3));
+                b[i] = make_float4(__ldcg(src + 16), __ldcg(src + 17), __ldcg(src + 18), __ldcg(src + 19));
+            }
         }
     }
 #pragma unroll
@@ -438,8 +445,10 @@ int lev_moe_gemm_run(lev_ctx* ctx, const lev_moe_weights* w, const float* x, int
     const int kc = job_tokens <= 64 ? 2 : 1, sms = ctx->prop.multiProcessorCount;
     for (int half = 0; half < 2; half++) {
         const lev_weights* t = half ? w->down : w->gate_up;
-        LEV_CUDA(ctx, launch_pdl(k_rows_f16, dim3((unsigned)pairs), dim3(128), (size_t)0, ctx->stream, half ? (const float*)act : x,
-                                 half ? (const int*)nullptr : perm, total_pos, top_k, (int)t->cols, half ? ah : xh, half ? as : xs));
+        const bool vec = half || ((uintptr_t)x & 15) == 0;   // columns are a multiple of 32: every row is aligned like the first
+        LEV_CUDA(ctx, launch_pdl(vec ? k_rows_f16<true> : k_rows_f16<false>, dim3((unsigned)pairs), dim3(128), (size_t)0, ctx->stream,
+                                 half ? (const float*)act : x, half ? (const int*)nullptr : perm, total_pos, top_k, (int)t->cols, half ? ah : xh,
+                                 half ? as : xs));
         ctx->launches++;
         LEV_TRY(lev_cuda_check(ctx, cudaGetLastError(), "k_rows_f16"));
         CUtensorMap map;

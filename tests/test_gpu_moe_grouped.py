@@ -93,3 +93,21 @@ def test_odd_numbers_of_stages(ctx, hidden, inter):
     x = torch.from_numpy(Q.normal(hidden, (260, hidden), 1.0)).cuda()
     check(ctx, layer, x, routing(rng, 260, 4, 32), times=8)
     layer.mw.free()
+
+
+@pytest.mark.parametrize("experts,hidden,inter,top_k,tokens", [(8, 256, 96, 4, 160), (16, 512, 128, 8, 64)])
+def test_activations_off_a_16_byte_boundary(ctx, experts, hidden, inter, top_k, tokens):
+    """A view that starts one float into its buffer, at 512 and 640 pairs: the job-list kernel does not take such rows, so
+    the grouped GEMM does."""
+    rng = np.random.default_rng(tokens)
+    layer = Layer(ctx, experts, hidden, inter, 7)
+    buf = torch.from_numpy(Q.normal(8, (tokens * hidden + 1,), 1.0)).cuda()
+    x = buf[1:].view(tokens, hidden)
+    assert x.data_ptr() % 16 == 4
+    idx = routing(rng, tokens, top_k, experts)
+    check(ctx, layer, x, idx)
+    out = ctx.moe_layer(layer.mw, x, top_k)
+    ref = ctx.moe_layer(layer.mw, x.clone(), top_k)
+    ctx.synchronize()
+    assert float((out - ref).norm() / ref.norm()) < 2e-3   # the aligned call may take the job-list kernel
+    layer.mw.free()
