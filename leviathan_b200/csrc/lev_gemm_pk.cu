@@ -278,13 +278,7 @@ __global__ void __launch_bounds__(PK_THREADS, 1) k_gemm_pk(const __grid_constant
             st.step(1);
         }
     }
-    __syncwarp();
-    if (*abort_flag) {
-        if (threadIdx.x == 0) atomicOr(A.status, LEV_DEV_TIMEOUT);
-        for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}   // copies in flight land before the CTA goes
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    pk_finish(abort_flag, A.status, LEV_DEV_TIMEOUT);
     if (CG == 2) cluster_sync_all();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == PK_MMA_WARP) {

@@ -304,13 +304,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) k_moe_gemm(const __grid_constan
             st.step(1);
         }
     }
-    __syncwarp();
-    if (*abort_flag) {
-        if (threadIdx.x == 0) atomicOr(A.status, LEV_DEV_TIMEOUT);
-        for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}   // copies in flight land before the CTA goes
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    pk_finish(abort_flag, A.status, LEV_DEV_TIMEOUT);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (warp == MG_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(512) : "memory");
 }

@@ -33,8 +33,6 @@ __device__ __forceinline__ unsigned pk_try(unsigned bar, unsigned parity) {
         : "memory");
     return ok;
 }
-// bounded wait; false on timeout or when another thread of the CTA has already given up.  The polls are spaced by
-// the loop's bookkeeping: a tight poll loop takes issue slots from the decode warps.
 // the same with the thread suspended for up to 20 us meanwhile: the polls of idle warps take issue slots otherwise
 __device__ __forceinline__ unsigned pk_try_suspended(unsigned bar, unsigned parity) {
     unsigned ok;
@@ -45,6 +43,7 @@ __device__ __forceinline__ unsigned pk_try_suspended(unsigned bar, unsigned pari
         : "memory");
     return ok;
 }
+// bounded wait (about a second); false on timeout or when another thread of the CTA has already given up
 __device__ __noinline__ bool pk_wait_slow(unsigned bar, unsigned parity, volatile int* abort_flag) {
     long long t_start = 0;
     for (unsigned i = 1;; i++) {
@@ -62,6 +61,16 @@ __device__ __noinline__ bool pk_wait_slow(unsigned bar, unsigned parity, volatil
 }
 __device__ __forceinline__ bool pk_wait(unsigned bar, unsigned parity, volatile int* abort_flag) {
     return pk_try(bar, parity) || pk_wait_slow(bar, parity, abort_flag);
+}
+// A CTA's last steps after its roles.  A thread that knows of a wait that ran out lets copies in flight land; the status
+// is set behind the barrier, because the warp that gave up may be the last to get here.
+__device__ __forceinline__ void pk_finish(volatile int* abort_flag, int* status, int bit) {
+    __syncwarp();
+    if (*abort_flag)
+        for (const long long t0 = clock64(); clock64() - t0 < 4000000LL;) {}
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(status, bit);
 }
 // ring position: stage and phase parity
 struct Ring {
