@@ -231,7 +231,14 @@ int lev_matvec_multi(lev_ctx* ctx, int n_ops, const lev_weights* const* w, const
  * Y[t][r] = sum_k bf16(W[r][k]) * X[t][k], f32 accumulate; X is bf16
  * [tokens][cols], Y is f32 [tokens][rows].  Replaces the act_f16 +
  * q4k/q6k_gemm_blocked_tokens program of
- * rust/crates/lev-forge/src/coopmat.rs:49-58, :236-425. */
+ * rust/crates/lev-forge/src/coopmat.rs:49-58, :236-425.
+ * Small outputs are cut along K, their partial products added in a fixed order: the same arguments give the
+ * same bits, eager and captured.  The partial products of an eager call lie in a buffer of the stream it runs
+ * on, those of a captured call in one that stays in place until lev_cuda_destroy: calls of up to 128 tokens of
+ * a 4-bit format share it among the context's graphs, which are therefore replayed one after another; longer
+ * and Q6_K calls have one per capture and stream.  A first call may be a captured one.  Where there is no
+ * buffer (from the fifth stream and the seventeenth captured prompt of a context on, or without memory) the
+ * call is not cut, takes longer and may differ in the last bits. */
 int lev_gemm_prefill(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int64_t tokens,
                      float* y, unsigned flags);
 /* f32 activations -> bf16 (round to nearest even); emit_act_f16's role

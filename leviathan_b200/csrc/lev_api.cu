@@ -140,6 +140,9 @@ extern "C" int lev_cuda_destroy(lev_ctx* ctx) {
     if (ctx->dist) lev_dist_destroy(ctx);
     for (int i = 0; i < LEV_SCR_SLOTS; i++)
         if (ctx->scratch[i]) cudaFree(ctx->scratch[i]);
+    for (int i = 0; i < ctx->split.eagers; i++) cudaFree(ctx->split.eager[i].p);
+    for (int i = 0; i < ctx->split.batches; i++) cudaFree(ctx->split.batch[i].p);
+    for (int i = 0; i < ctx->split.prompts; i++) cudaFree(ctx->split.prompt[i].p);
     cudaFree(ctx->d_status);
     if (ctx->chain_sync) cudaFree(ctx->chain_sync);
     cudaFreeHost(ctx->h_status);

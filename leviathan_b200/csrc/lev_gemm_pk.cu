@@ -365,6 +365,60 @@ int launch_pk(lev_ctx* ctx, const CUtensorMap& map, const PkArgs& A, int grid, s
     return LEV_OK;
 }
 
+// Allocations that may happen beside a stream capture (of this call or of another thread): cudaMalloc is no stream
+// operation and legal there, but a capture in global mode has it refused unless the thread says that it knows.
+struct CaptureRelaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureRelaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+bool split_alloc(lev_split_buffer* b, unsigned long long stream, unsigned long long capture, size_t bytes) {
+    *b = {stream, capture, nullptr, 0};
+    const CaptureRelaxed relaxed;
+    if (cudaMalloc(&b->p, bytes) != cudaSuccess) return false;
+    b->bytes = bytes;
+    return true;
+}
+
+// The buffer of a call's partial products, or NULL: the call is then planned without a split.
+float* split_buffer(lev_ctx* ctx, size_t bytes, bool prompt) {
+    lev_split_buffers& B = ctx->split;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long stream = (unsigned long long)(uintptr_t)ctx->stream, capture = 0;
+    if (cudaStreamGetCaptureInfo(ctx->stream, &cs, &capture) != cudaSuccess) return nullptr;
+    if (cs == cudaStreamCaptureStatusNone) {
+        {
+            const CaptureRelaxed relaxed;   // the id is not to be had from a stream that is being captured
+            if (cudaStreamGetId(ctx->stream, &stream) != cudaSuccess) return nullptr;
+        }
+        lev_split_buffer* b = B.eager;
+        while (b < B.eager + B.eagers && b->stream != stream) b++;
+        if (b == B.eager + LEV_SPLIT_EAGER) return nullptr;
+        if (b == B.eager + B.eagers) {
+            if (!split_alloc(b, stream, 0, bytes + bytes / 4)) return nullptr;
+            B.eagers++;
+        } else if (b->bytes < bytes) {   // grows; only this stream's calls use it
+            const CaptureRelaxed relaxed;
+            if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return nullptr;
+            cudaFree(b->p);
+            if (!split_alloc(b, stream, 0, bytes + bytes / 4)) return nullptr;
+        }
+        return (float*)b->p;
+    }
+    lev_split_buffer* list = prompt ? B.prompt : B.batch;
+    int& n = prompt ? B.prompts : B.batches;
+    size_t most = 0;
+    for (int i = n - 1; i >= 0; i--)
+        if (!prompt || (list[i].stream == stream && list[i].capture == capture)) {
+            if (list[i].bytes >= bytes) return (float*)list[i].p;
+            most = list[i].bytes > most ? list[i].bytes : most;
+        }
+    if (n == (prompt ? LEV_SPLIT_PROMPT : LEV_SPLIT_BATCH) || !split_alloc(&list[n], stream, capture, bytes > 2 * most ? bytes : 2 * most))
+        return nullptr;
+    return (float*)list[n++].p;
+}
+
 }  // namespace
 
 // shapes the tensor-memory kernel serves: repacked tensors, activations on a 16-byte boundary
@@ -379,13 +433,11 @@ int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int6
     const int64_t kt = (w->cols + PK_KS - 1) / PK_KS;
     const bool can_split = ((uintptr_t)y & 15) == 0 && (tokens * w->rows) % 4 == 0;
     PkPlan P = pk_plan(ctx, w->type, w->rows, kt, tokens, can_split);
-    if (P.splits > 1 && (tokens > 128 || w->type == LEV_GGML_Q6_K)) {
-        // A captured call of prompt size keeps to the caller's buffers: partial products would need scratch that cannot
-        // grow inside a capture, and the graph would hold its address.  (Decode batches of the 4-bit formats split there
-        // too: their callers run the step once before they capture it.)
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        LEV_CUDA(ctx, cudaStreamIsCapturing(ctx->stream, &cs));
-        if (cs != cudaStreamCaptureStatusNone) P = pk_plan(ctx, w->type, w->rows, kt, tokens, false);
+    // Captured calls split like eager ones (the same bits): the buffer is one that graphs may hold.
+    float* part = nullptr;
+    if (P.splits > 1 && !(part = split_buffer(ctx, (size_t)P.splits * tokens * w->rows * sizeof(float), tokens > 128 || w->type == LEV_GGML_Q6_K))) {
+        cudaGetLastError();   // out of memory is no error of this call
+        P = pk_plan(ctx, w->type, w->rows, kt, tokens, false);
     }
     CUtensorMap map;
     const cuuint64_t gdim[2] = {(cuuint64_t)w->cols, (cuuint64_t)tokens};
@@ -411,13 +463,8 @@ int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int6
     A.parts = P.parts;
     A.stages = P.stages;
     A.acc_stages = P.n_part * P.parts <= 256 ? 2 : 1;
-    A.y = y;
+    A.y = part ? part : y;
     A.status = ctx->d_status;
-    if (P.splits > 1) {
-        void* scr;
-        LEV_TRY(lev_scratch(ctx, LEV_SCR_GEMM, (size_t)P.splits * tokens * w->rows * sizeof(float), &scr));
-        A.y = (float*)scr;
-    }
     const int64_t tiles = (int64_t)A.row_tiles * A.splits * A.tok_tiles;
     const int grid = (int)(tiles < P.units ? tiles : P.units) * P.cg;
     int st;
@@ -432,11 +479,11 @@ int lev_gemm_tc_run(lev_ctx* ctx, const lev_weights* w, const void* x_bf16, int6
     if (st) return st;
     ctx->launches++;
     LEV_TRY(lev_cuda_check(ctx, cudaGetLastError(), "k_gemm_pk"));
-    if (P.splits > 1) {
+    if (part) {
         const int64_t n4 = tokens * w->rows / 4;
         const int64_t blocks = (n4 + 255) / 256, cap = (int64_t)ctx->prop.multiProcessorCount * 8;
         LEV_CUDA(ctx, launch_pdl(k_gemm_split_sum, dim3((unsigned)(blocks < cap ? blocks : cap)), dim3(256), (size_t)0, ctx->stream,
-                                 (const float4*)A.y, P.splits, n4, (float4*)y));
+                                 (const float4*)part, P.splits, n4, (float4*)y));
         ctx->launches++;
         return lev_cuda_check(ctx, cudaGetLastError(), "k_gemm_split_sum");
     }

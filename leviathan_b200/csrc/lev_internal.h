@@ -34,6 +34,21 @@
 
 struct lev_dist_state;
 
+// Partial products of K-split GEMMs (lev_gemm_pk.cu) lie outside the scratch slots: products on different streams must
+// not meet in one buffer, and a buffer whose address a graph holds must neither move nor be written by eager calls.
+#define LEV_SPLIT_EAGER 4      // eager calls: one growing buffer for each of a context's first streams
+#define LEV_SPLIT_BATCH 40     // captured decode batches share one; a larger one (at least twice) replaces it for later captures
+#define LEV_SPLIT_PROMPT 16    // captured prompts: one per capture and stream
+struct lev_split_buffer {
+    unsigned long long stream, capture;   // eager: the stream's id (handles are used again); captured: handle and capture id
+    void* p;
+    size_t bytes;
+};
+struct lev_split_buffers {
+    lev_split_buffer eager[LEV_SPLIT_EAGER], batch[LEV_SPLIT_BATCH], prompt[LEV_SPLIT_PROMPT];
+    int eagers, batches, prompts;
+};
+
 struct lev_ctx {
     int device;
     cudaStream_t own_stream;
@@ -45,6 +60,7 @@ struct lev_ctx {
     // scratch owned by the context, grown on demand, reused across calls
     void* scratch[12];
     size_t scratch_bytes[12];
+    lev_split_buffers split;
     int* d_status;   // device status word
     int* h_status;   // pinned mirror
     cudaEvent_t ev0, ev1;
@@ -67,7 +83,6 @@ enum {
     LEV_SCR_XPREP = 6,   // split activations for the stream schedule
     LEV_SCR_DIST = 7,
     LEV_SCR_ATTN = 8,    // attention partials per position range
-    LEV_SCR_GEMM = 9,    // partial products of a K-split prefill GEMM
     LEV_SCR_SLOTS = 12
 };
 
