@@ -602,13 +602,15 @@ bool dense_plan_tiles(lev_ctx* ctx, const lev_weights* w, int64_t tiles, int n_c
     size_t cap = (size_t)110 * 1024;
     if (n_cols > 4) {
         // Five to eight columns: the tables leave no room for a second CTA, so one takes the SM, with as many warps as
-        // keep two K-steps each in flight (16 up to 3900 columns of K at eight columns).  Served from tables in global memory
-        // behind a preparation launch (k_prepare_x, k_stream) the same calls took: [12288 x 4096] Q4_K 21.2 / 23.9 us at
-        // five / eight columns, 17.7 / 19.9 here; [4096 x 2816] Q4_0 at six 16.7, 9.8 here; [16384 x 2048] Q6_K at five
-        // 23.9, 15.2 here; [512 x 1024] Q4_0 at eight 15.3, 5.3 here.  Of 13 shapes from 200 x 320 to 65536 x 2816 none
-        // was slower.
+        // keep two K-steps each in flight (at eight columns 16 up to 3840 columns of K in the 4-bit formats and 2816 in
+        // Q6_K).  Served from tables in global memory behind a preparation launch (k_prepare_x, k_stream) the same calls
+        // took, back to back: [24576 x 4096] Q4_K at eight columns 35.9 us, 31.0 here; [12288 x 4096] at five / eight 20.9 /
+        // 23.3, 18.1 / 20.1 here; [4096 x 2816] Q4_0 at six 16.7, 9.7 here; [65536 x 2816] Q6_K at five 76.2, 54.6 here;
+        // [512 x 1024] Q4_0 at eight 15.1, 5.1 here.  With eight warps Q4_K is the slower one ([28672 x 5632] at seven
+        // columns 49.5 us, 56.6 here; [8192 x 7680] at five 24.3, 27.1 here), Q4_0 (56.4, 53.7 here) and Q6_K are not.
         cap = 200 * 1024;
         warps = tb + 16 * 2 * step <= cap ? 16 : tb + 12 * 2 * step <= cap ? 12 : 8;
+        if (warps == 8 && w->type == LEV_GGML_Q4_K) return false;
         if (tb + 8 * 2 * step > cap) return false;
     }
     const int sms = ctx->prop.multiProcessorCount;
@@ -760,6 +762,7 @@ int lev_dense_run(lev_ctx* ctx, const lev_weights* w, int64_t row0, int64_t rows
                                         : launch_dense_c<LEV_GGML_Q4_0>(ctx, n_cols, P.warps, P.grid, P.smem, A);
     if (st) return st;
     ctx->launches++;
+    if (n_cols > 4) ctx->full_dense_at = ctx->launches;
     ctx->ev.grid = P.grid;
     ctx->ev.block = P.warps * 32;
     return lev_cuda_check(ctx, cudaGetLastError(), "k_dense");

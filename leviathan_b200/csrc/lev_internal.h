@@ -56,6 +56,7 @@ struct lev_ctx {
     cudaDeviceProp prop;
     char err[512];
     int64_t launches;
+    int64_t full_dense_at;   // `launches` behind the last one-launch product of more than four columns (lev_dense.cu)
     lev_evidence ev;
     // scratch owned by the context, grown on demand, reused across calls
     void* scratch[12];

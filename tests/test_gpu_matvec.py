@@ -366,3 +366,30 @@ def test_five_to_eight_columns_in_one_launch(ctx, name, n_cols, rows, cols):
     for c in range(n_cols):
         assert O.max_rel_err(y[c].cpu().numpy(), O.matvec_f64(t, w, rows, cols, x[c])) < H.REPORT_TOL
     wh.free()
+
+
+@pytest.mark.parametrize("name,n_cols,cols,launches", [
+    ("q4_k", 7, 5120, 1), ("q4_k", 7, 5632, 2), ("q4_k", 8, 4864, 2),   # Q4_K: up to the last size with twelve warps
+    ("q4_0", 7, 5632, 1), ("q6_k", 8, 4096, 1), ("q6_k", 6, 5632, 2),
+])
+def test_route_of_five_to_eight_columns(ctx, name, n_cols, cols, launches):
+    """One launch where enough warps have room beside the tables, else the preparation and the stream kernel; either way
+    the same calls in turn with a two-launch one, whose preparation is launched plainly, give their own results."""
+    t = H.TYPES[name]
+    w = H.quantized(t, 61, 160, cols)
+    wide = H.quantized(H.TYPES["q6_k"], 62, 48, 12288)
+    x, xw = Q.normal(63, (n_cols, cols), 1.0), Q.normal(64, (n_cols, 12288), 1.0)
+    wh, wwh = ctx.upload(w, t, 160, cols), ctx.upload(wide, H.TYPES["q6_k"], 48, 12288)
+    dx, dxw = torch.from_numpy(x).cuda(), torch.from_numpy(xw).cuda()
+    l0 = ctx.launch_count()
+    y = ctx.matvec(wh, dx)
+    assert ctx.launch_count() - l0 == launches
+    for _ in range(3):
+        yw, y2 = ctx.matvec(wwh, dxw), ctx.matvec(wh, dx)
+        ctx.synchronize()
+        assert torch.equal(y, y2)
+    for c in (0, n_cols - 1):
+        assert O.max_rel_err(y[c].cpu().numpy(), O.matvec_f64(t, w, 160, cols, x[c])) < H.REPORT_TOL
+        assert O.max_rel_err(yw[c].cpu().numpy(), O.matvec_f64(H.TYPES["q6_k"], wide, 48, 12288, xw[c])) < H.REPORT_TOL
+    wh.free()
+    wwh.free()
