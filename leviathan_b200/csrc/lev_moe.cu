@@ -769,8 +769,10 @@ __global__ void __launch_bounds__(1024) k_group_fast(GroupArgs G, int nchunks) {
 // out[t][h] = sum_k w[t][k] * y[t][k][h]: a separate multiply and add per
 // slot in rank order from zero (Sources/LeviathanCore/Gemma4.swift:4459-4466)
 // residual != NULL: out = residual + alpha * sum, the bits of lev_axpy applied to the plain sum (out may be residual)
-// blockIdx.y: token (grid-stride); V: elements per thread (four where rows are 16-byte aligned: 16.6 -> 11.3 us at 512
-// tokens of 2816, where eight rows of f32 per token are 46 MB out of L2)
+// blockIdx.y: token (grid-stride); V: elements per thread.  Four, where rows are 16-byte aligned and there is work for it:
+// one element per thread took 12.6 us at 512 tokens of 2816 (eight rows of f32 per token, 46 MB out of L2), four take 6.4.
+// Few elements are a matter of latency, where single loads win: 1.28 us against 1.54 at one token, 1.46 against 1.64 at
+// eight; the two meet near two blocks of single elements per SM (13 tokens of 2816; back to back in a graph).
 template <int V>
 __global__ void __launch_bounds__(128) k_combine(const float* __restrict__ y, const float* __restrict__ w, int64_t tokens, int top_k,
                                                  int hidden, float* out, const int32_t* __restrict__ idx, int first, int count,
@@ -1207,7 +1209,8 @@ int lev_moe_combine_resident_dev(lev_ctx* ctx, const float* y, const float* wts,
 
 int lev_moe_combine_residual_dev(lev_ctx* ctx, const float* y, const float* wts, int64_t tokens, int top_k, int hidden,
                                  float* out, const int32_t* idx, int first, int count, const float* residual, float alpha) {
-    const bool vec = hidden % 4 == 0 && (((uintptr_t)y | (uintptr_t)out | (uintptr_t)residual) & 15) == 0;
+    const bool vec = tokens * hidden > (int64_t)ctx->prop.multiProcessorCount * 256 && hidden % 4 == 0 &&
+                     (((uintptr_t)y | (uintptr_t)out | (uintptr_t)residual) & 15) == 0;
     const dim3 grid((unsigned)((hidden + (vec ? 511 : 127)) / (vec ? 512 : 128)), (unsigned)(tokens < 65535 ? tokens : 65535));
     LEV_CUDA(ctx, launch_pdl(vec ? k_combine<4> : k_combine<1>, grid, dim3(128), (size_t)0, ctx->stream, y, wts, tokens, top_k, hidden, out, idx,
                              first, count, residual, alpha));

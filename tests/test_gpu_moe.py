@@ -156,6 +156,22 @@ def test_combine_is_rank_ordered(ctx):
     assert e.value.name == "nonFiniteInput"
 
 
+@pytest.mark.parametrize("tokens,top_k,hidden", [(1, 8, 2816), (3, 3, 1056), (37, 8, 1024), (38, 8, 1024), (9, 9, 4128), (70, 1, 601), (5, 17, 8192)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_combine_forms(ctx, tokens, top_k, hidden, shift):
+    """Single elements and four per thread (from two blocks of single ones per SM on: 37888 outputs of 148 SMs), ragged
+    widths, rows off a 16-byte boundary: the oracle's bits."""
+    rng = np.random.default_rng(tokens + hidden)
+    y = torch.empty(tokens * top_k * hidden + shift, device="cuda")[shift:].view(tokens, top_k, hidden)
+    y.copy_(torch.from_numpy(rng.standard_normal((tokens, top_k, hidden)).astype(np.float32)))
+    w = rng.random((tokens, top_k)).astype(np.float32)
+    l0 = ctx.launch_count()
+    out = ctx.moe_combine(y, torch.from_numpy(w).cuda()).cpu().numpy()
+    assert ctx.launch_count() - l0 == 1
+    for t in sorted({0, tokens // 2, tokens - 1}):
+        assert np.array_equal(out[t].view(np.uint32), O.combine(y[t].cpu().numpy(), w[t]).view(np.uint32))
+
+
 @pytest.mark.parametrize("name,tokens", [("tail", 4), ("lanes", 3), ("gemma", 1), ("gemma", 32)])
 def test_layer_matches_oracle(ctx, models, name, tokens):
     m = models[name]
