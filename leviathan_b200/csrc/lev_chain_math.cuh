@@ -49,7 +49,7 @@ __device__ __forceinline__ void mma0(float* d, unsigned a0, unsigned a1, unsigne
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// u8 x s8 products of 32 columns, exact in 32-bit integers; the second form starts from zero
+// products of 32 columns with s8 digits, exact in 32-bit integers: weights u8 or s8; the forms with a 0 start from zero
 __device__ __forceinline__ void imma(int* d, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
         : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
@@ -60,6 +60,19 @@ __device__ __forceinline__ void imma0(int* d, unsigned a0, unsigned a1, unsigned
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
 }
+__device__ __forceinline__ void imma_s8(int* d, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void imma0_s8(int* d, unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+// 16 (q - 8) of the high / low nibbles q of four bytes, as signed bytes
+__device__ __forceinline__ unsigned high_s8(unsigned w) { return (w & 0xF0F0F0F0u) ^ 0x80808080u; }
+__device__ __forceinline__ unsigned low_s8(unsigned w) { return ((w << 4) & 0xF0F0F0F0u) ^ 0x80808080u; }
 // byte k of w divided by 16, as a float: 2^19 + byte / 16, minus 2^19
 __device__ __forceinline__ float byte_to_float_16th(unsigned w, unsigned k) {
     return __uint_as_float(__byte_perm(w, 0x49000000u, 0x7650u + k)) - 524288.0f;
@@ -76,12 +89,12 @@ __device__ __forceinline__ float byte_to_float_16th(unsigned w, unsigned k) {
 // 32.3 -> 30.2 us, [12288 x 6144] Q4_K 14.7 -> 13.4 us.  lev_dense.cu stays with the f16 form: job lists of one column gained
 // nothing (28.2 against 27.7 us for a MoE layer of one token, where two processes of one build differ by 1.5 %: the tables
 // cost what a short share wins back), and plain products agree with their wider calls there.
-// Table of a K-step: fragments [chunk][digit][quad lane][four mma registers] (1 KB), then kIntAux bytes of sums:
-// Q4_K: activation sums of the eight sub-blocks (f32), Q4_0: -8 * (digit sum) [chunk][digit / 2][block][digit & 1] (s32);
-// then the power of two (f32; NaN where an activation is not finite, so that the results are).
+// Table of a K-step: fragments [chunk][digit][quad lane][four mma registers] (1 KB); after all fragments kOneColAux bytes
+// per K-step: Q4_K: activation sums of the eight sub-blocks (f32); then, both, the power of two (f32; NaN where an
+// activation is not finite, so that the results are).  Q4_0 needs no sums: its products take q - 8 as it is.
 // ---------------------------------------------------------------------------
 template <int TYPE>
-constexpr unsigned kOneColAux = TYPE == LEV_GGML_Q4_K ? 48u : TYPE == LEV_GGML_Q6_K ? 128u : 144u;   // per K-step
+constexpr unsigned kOneColAux = TYPE == LEV_GGML_Q4_K ? 40u : TYPE == LEV_GGML_Q6_K ? 128u : 8u;
 constexpr unsigned kZeroBytes = 528;   // zeros that stand in for the fragments of the other parity
 
 // Builds the entries of one (chunk, quad lane): v[m] are the four activations of mma register m (chunk_col order).
@@ -134,26 +147,9 @@ __device__ __forceinline__ bool int_tables(const float4* v, int chunk, int tt, b
             s += __shfl_xor_sync(0xffffffffu, s, 2);
             if (live && tt == 0) reinterpret_cast<float*>(mine)[c * 2 + hf] = s;
         }
-    } else {
-        // digit sums of the chunk's two blocks, two digits to a word: |sum| <= 4096
-        int s[2][2];
-#pragma unroll
-        for (int b = 0; b < 2; b++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int lo = __dp4a((int)T[2 * b][2 * h], 0x01010101, __dp4a((int)T[2 * b + 1][2 * h], 0x01010101, 0));
-                const int hi = __dp4a((int)T[2 * b][2 * h + 1], 0x01010101, __dp4a((int)T[2 * b + 1][2 * h + 1], 0x01010101, 0));
-                int p = lo + hi * 65536;
-                p += __shfl_xor_sync(0xffffffffu, p, 1);
-                p += __shfl_xor_sync(0xffffffffu, p, 2);
-                s[h][b] = p;
-            }
-        const int p = tt & 2 ? (tt & 1 ? s[1][1] : s[1][0]) : (tt & 1 ? s[0][1] : s[0][0]);
-        const int lo = (int)(short)(p & 0xffff), hi = (p - lo) >> 16;
-        if (live) reinterpret_cast<int2*>(mine)[c * 4 + tt] = make_int2(-8 * lo, -8 * hi);
     }
     if (live && c == 0 && tt == 0)
-        *reinterpret_cast<float*>(mine + kOneColAux<TYPE> - 16) = most >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((unsigned)(97 + e) << 23);
+        *reinterpret_cast<float*>(mine + kOneColAux<TYPE> - 8) = most >= 0x7f800000u ? __uint_as_float(0x7fc00000u) : __uint_as_float((unsigned)(97 + e) << 23);
     return bad && live;
 }
 
@@ -357,19 +353,23 @@ __device__ __forceinline__ void int_step(unsigned st, unsigned xk, unsigned ak, 
         ya = fmaf(scale * h2f_bits(h0.x & 0xffffu), pa, fmaf(-dminA, qa, ya));
         yb = fmaf(scale * h2f_bits(h1.x & 0xffffu), pb, fmaf(-dminB, qb, yb));
     } else {
-        // Q4_0: accumulators [chunk pair][block], starting at -8 times the digit sums
-        const float scale = __uint_as_float(lds32(ak + 128)) * L.place;
+        // Q4_0: accumulators [chunk pair][block], 16 times the sums
+        const float scale = __uint_as_float(lds32(ak)) * (0.0625f * L.place);
         const unsigned own = L.t >> 1;   // this lane holds two digits of chunk own (pair 0) and 2 + own (pair 1)
 #pragma unroll
         for (int p = 0; p < 2; p++) {
-            const uint4 kk = lds128(ak + 64 * p + 16 * t);
-            int acc[2][4] = {{(int)kk.x, (int)kk.y, (int)kk.x, (int)kk.y}, {(int)kk.z, (int)kk.w, (int)kk.z, (int)kk.w}};
+            int acc[2][4];
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const uint4 q = lds128(st + (2 * p + j) * 576 + 64 + L.q_off);
                 const uint4 x = lds128((j ? odd : even) + p * 512);
-                imma(acc[0], q.x & 0x0F0F0F0Fu, q.z & 0x0F0F0F0Fu, (q.x >> 4) & 0x0F0F0F0Fu, (q.z >> 4) & 0x0F0F0F0Fu, x.x, x.y);
-                imma(acc[1], q.y & 0x0F0F0F0Fu, q.w & 0x0F0F0F0Fu, (q.y >> 4) & 0x0F0F0F0Fu, (q.w >> 4) & 0x0F0F0F0Fu, x.z, x.w);
+                if (j) {
+                    imma_s8(acc[0], low_s8(q.x), low_s8(q.z), high_s8(q.x), high_s8(q.z), x.x, x.y);
+                    imma_s8(acc[1], low_s8(q.y), low_s8(q.w), high_s8(q.y), high_s8(q.w), x.z, x.w);
+                } else {
+                    imma0_s8(acc[0], low_s8(q.x), low_s8(q.z), high_s8(q.x), high_s8(q.z), x.x, x.y);
+                    imma0_s8(acc[1], low_s8(q.y), low_s8(q.w), high_s8(q.y), high_s8(q.w), x.z, x.w);
+                }
             }
             // fp16 d of (row g, blk 0 | blk 1), (row g+8, ...) of the chunk
             const uint2 sc = lds64(st + (2 * p + own) * 576 + 8 * L.g);

@@ -71,6 +71,7 @@ struct lev_ctx {
     void* chain_sync;
     void* chain_part;
     int chain_off, chain_warps, chain_depth;
+    size_t chain_static[2];   // static shared memory of its forms with 16 and 12 compute warps
 };
 
 // Scratch slots (each one buffer; a call may use several at once).

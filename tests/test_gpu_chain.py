@@ -246,3 +246,27 @@ def test_integer_activations_not_finite(ctx, name):
         out = ctx.matvec_chain([dict(w=wh, x=_dev(x), out=torch.empty(40, device="cuda"))])[0]
         assert not bool(torch.isfinite(out).any())
         wh.free()
+
+
+@pytest.mark.parametrize("gate,down,hidden,inter", [
+    ("q4_k", "q6_k", 8192, 16384), ("q4_0", "q4_0", 7168, 16384), ("q6_k", "q4_0", 8192, 16384),   # the longest, twelve compute warps
+    ("q4_0", "q4_0", 1024, 13952), ("q4_0", "q4_0", 1024, 8192), ("q4_k", "q6_k", 1536, 13824),    # short rings: twelve, sixteen, sixteen
+])
+def test_long_activations_fit_one_launch(ctx, gate, down, hidden, inter):
+    """The activation tables of both halves of an FFN beside the rings: the longest lists that one launch holds."""
+    x, a = Q.normal(71, (hidden,), 1.0), Q.normal(72, (inter,), 1.0)
+    dx, da = _dev(x), _dev(a)
+    ops, refs, handles = [], [], []
+    for i, (name, cols, vec, dev) in enumerate(((gate, hidden, x, dx), (gate, hidden, x, dx), (down, inter, a, da))):
+        w = H.quantized(H.TYPES[name], 73 + i, 40, cols)
+        handles.append(ctx.upload(w, H.TYPES[name], 40, cols))
+        refs.append(O.matvec_f64(H.TYPES[name], w, 40, cols, vec))
+        ops.append(dict(w=handles[-1], x=dev, out=torch.empty(40, device="cuda")))
+    l0 = ctx.launch_count()
+    outs = ctx.matvec_chain(ops)
+    assert ctx.launch_count() - l0 == 1
+    ctx.synchronize()
+    for out, ref in zip(outs, refs):
+        assert O.max_rel_err(out.cpu().numpy(), ref) < H.REPORT_TOL
+    for h in handles:
+        h.free()
