@@ -1096,7 +1096,7 @@ static int experts_dev_impl(lev_ctx* ctx, const lev_moe_weights* w, const float*
     const int64_t min_pairs = 512;
     const bool tensor = !sliced && !sliced4_early && pairs >= min_pairs && lev_moe_gemm_supported(w);
     const bool sliced4 = sliced4_early || (!sliced && !tensor && moe_sliced4(ctx, w, pairs, x));
-    const int cmax = sliced ? 1 : tensor ? lev_moe_gemm_job_tokens(pairs, w->local_count) : sliced4 ? 4 : (pairs <= 2 * (int64_t)w->local_count ? 4 : 8), terms = 2;
+    const int cmax = sliced ? 1 : tensor ? lev_moe_gemm_job_tokens(pairs, w->experts) : sliced4 ? 4 : (pairs <= 2 * (int64_t)w->local_count ? 4 : 8), terms = 2;
     int64_t mj = (int64_t)w->local_count + pairs / cmax;
     if (mj > pairs) mj = pairs;
     const int max_jobs = (int)mj;

@@ -404,7 +404,7 @@ int launch_mg(lev_ctx* ctx, const CUtensorMap& map, const MgArgs& A, int grid, s
 }  // namespace
 
 // Tokens of a job: 64 with two chunks per stage while an expert's share mostly fits that (a Poisson share of 40 exceeds
-// 64 once in ten thousand), else 256 (one accumulator of two).
+// 64 once in ten thousand), else 256 (one accumulator of two).  The pairs are those of all experts, resident or not.
 int lev_moe_gemm_job_tokens(int64_t pairs, int experts) { return pairs <= 40 * (int64_t)experts ? 64 : 256; }
 
 bool lev_moe_gemm_supported(const lev_moe_weights* w) {

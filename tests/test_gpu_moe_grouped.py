@@ -111,3 +111,24 @@ def test_activations_off_a_16_byte_boundary(ctx, experts, hidden, inter, top_k, 
     ctx.synchronize()
     assert float((out - ref).norm() / ref.norm()) < 2e-3   # the aligned call may take the job-list kernel
     layer.mw.free()
+
+
+@pytest.mark.parametrize("first,count", [(0, 8), (24, 8), (12, 4)])
+def test_resident_experts_only(ctx, first, count):
+    """A rank's share of the experts at a prefill-sized call: its pairs, nothing else, and the jobs are sized by an
+    expert's share of all pairs."""
+    rng = np.random.default_rng(first)
+    e, h, i = 32, 640, 192
+    layer = Layer(ctx, e, h, i, 300 + first)
+    gs, ds = 2 * i * (h // 32) * 18, h * (i // 32) * 18
+    part = ctx.moe_upload(layer.rw, layer.gu[first * gs:(first + count) * gs], layer.dn[first * ds:(first + count) * ds], e, h, i,
+                          local_first=first, local_count=count)
+    x = torch.from_numpy(Q.normal(31, (256, h), 1.0)).cuda()
+    idx = routing(rng, 256, 4, e)
+    mine = ((idx >= first) & (idx < first + count))
+    y = ctx.moe_experts(part, x, idx)
+    ctx.synchronize()
+    want, bound, _, _ = reference(layer, x, idx)
+    assert bool(((y.double() - want).abs() <= bound)[mine].all())
+    part.free()
+    layer.mw.free()
