@@ -6,11 +6,13 @@ PyTorch fallback for any operation of this package.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "lib", "libleviathan_cuda.so")
-HOST_PATH = os.path.join(HERE, "lib", "_pyhost.so")
+HOST_PATH = os.path.join(HERE, "lib", "_pyhost" + importlib.machinery.EXTENSION_SUFFIXES[0])   # one per interpreter
 
 # status codes (include/leviathan_cuda.h, enum lev_status)
 OK = 0
@@ -174,19 +176,39 @@ def load() -> C.CDLL:
     return lib
 
 
+class _CtypesHost:
+    """The calls of csrc/lev_pyhost.c through ctypes, for an interpreter it is not built for: the same arguments, a
+    microsecond or two more per call."""
+
+    def __init__(self, lib: C.CDLL):
+        self._lib = lib
+        for name in ("matvec", "rmsnorm", "axpy", "act_bf16", "gemm_prefill", "moe_layer", "moe_layer_residual"):
+            setattr(self, name, getattr(lib, "lev_" + name))
+
+    def matvec_fused(self, ctx, w, row0, rows, x, x_count, n_cols, prologue, norm_weight, eps, residual, alpha, y, cap):
+        f = Fusion(prologue, norm_weight, eps, residual, alpha)
+        return self._lib.lev_matvec_fused(ctx, w, row0, rows, x, x_count, n_cols, C.byref(f), y, cap)
+
+    def matvec_chain(self, ctx, n, ops, flags):
+        return self._lib.lev_matvec_chain(ctx, n, C.cast(ops, C.POINTER(ChainOp)), flags)
+
+    def kv_append(self, ctx, layout, *args):
+        return self._lib.lev_kv_append(ctx, C.cast(layout, C.POINTER(KVLayout)), *args)
+
+    def attn_decode(self, ctx, layout, *args):
+        return self._lib.lev_attn_decode(ctx, C.cast(layout, C.POINTER(KVLayout)), *args)
+
+
 def host():
     """The native calls of csrc/lev_pyhost.c: the same entry points for the calls made per token, without ctypes'
-    argument conversion.  Raises if it is not built, like load()."""
+    argument conversion; through ctypes where they are not built for this interpreter."""
     global _host
     if _host is None:
-        load()
-        if not os.path.exists(HOST_PATH):
-            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m leviathan_b200.build`")
-        import importlib.machinery
-        import importlib.util
-
-        loader = importlib.machinery.ExtensionFileLoader("_pyhost", HOST_PATH)
-        spec = importlib.util.spec_from_loader("_pyhost", loader)
-        _host = importlib.util.module_from_spec(spec)
-        loader.exec_module(_host)
+        lib = load()
+        if os.path.exists(HOST_PATH):
+            loader = importlib.machinery.ExtensionFileLoader("_pyhost", HOST_PATH)
+            _host = importlib.util.module_from_spec(importlib.util.spec_from_loader("_pyhost", loader))
+            loader.exec_module(_host)
+        else:
+            _host = _CtypesHost(lib)
     return _host

@@ -11,13 +11,14 @@ import os
 import subprocess
 import sys
 import sysconfig
+from importlib.machinery import EXTENSION_SUFFIXES
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libleviathan_cuda.so")
-HOST_PATH = os.path.join(LIB_DIR, "_pyhost.so")
+HOST_PATH = os.path.join(LIB_DIR, "_pyhost" + EXTENSION_SUFFIXES[0])
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -68,12 +69,18 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
         cmd = [nvcc, "-shared", "-cudart", "static", "-gencode", "arch=compute_100a,code=sm_100a",
                "-o", LIB_PATH, *objects, "-ldl", "-lpthread"]
         subprocess.run(cmd, check=True)
-    # the native calls of the Python layer (csrc/lev_pyhost.c), bound to the library beside it
+    # The native calls of the Python layer (csrc/lev_pyhost.c) for this interpreter, bound to the library beside them.
+    # Without a C compiler or Python's headers the package goes through ctypes.
     src = os.path.join(CSRC, "lev_pyhost.c")
     if force or _stale(HOST_PATH, [src, LIB_PATH] + headers):
-        subprocess.run([os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", os.path.join(ROOT, "include"),
-                        "-I", sysconfig.get_paths()["include"], "-o", HOST_PATH, src, "-L", LIB_DIR, "-l:libleviathan_cuda.so",
-                        "-Wl,-rpath,$ORIGIN"], check=True)
+        cmd = [os.environ.get("CC", "gcc"), "-O2", "-Wall", "-shared", "-fPIC", "-I", os.path.join(ROOT, "include"),
+               "-I", sysconfig.get_paths()["include"], "-o", HOST_PATH, src, "-L", LIB_DIR, "-l:libleviathan_cuda.so", "-Wl,-rpath,$ORIGIN"]
+        try:
+            subprocess.run(cmd, check=True)
+        except (OSError, subprocess.CalledProcessError) as e:
+            if os.path.exists(HOST_PATH):
+                os.remove(HOST_PATH)
+            print(f"lev_pyhost.c is not built ({e}): calls go through ctypes", file=sys.stderr)
     return LIB_PATH
 
 

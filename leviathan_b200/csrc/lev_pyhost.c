@@ -36,7 +36,6 @@ static float F(PyObject* o) { return (float)PyFloat_AsDouble(o); }
         return PyLong_FromLong(st);                                                                       \
     }
 
-HOST_FN(set_stream, 2, lev_ctx* c = P(a[0]); void* s = P(a[1]), lev_cuda_set_stream(c, s))
 HOST_FN(matvec, 11, lev_ctx* c = P(a[0]); lev_weights* w = P(a[1]); long long r0 = I(a[2]); long long rows = I(a[3]); float* x = P(a[4]);
         long long xc = I(a[5]); long long nc = I(a[6]); float* y = P(a[7]); long long cap = I(a[8]); long long sched = I(a[9]); long long fl = I(a[10]),
         lev_matvec(c, w, r0, rows, x, xc, (int)nc, y, cap, (int)sched, (unsigned)fl))
@@ -67,7 +66,7 @@ HOST_FN(attn_decode, 13, lev_ctx* c = P(a[0]); lev_kv_layout* l = P(a[1]); void*
         float sc = F(a[11]); float* y = P(a[12]), lev_attn_decode(c, l, kp, vp, tb, s, p, (int)nc, (int)qh, q, (int)win, sc, y))
 
 #define ENTRY(NAME) {#NAME, (PyCFunction)(void (*)(void))NAME, METH_FASTCALL, NULL}
-static PyMethodDef methods[] = {ENTRY(set_stream), ENTRY(matvec), ENTRY(matvec_fused), ENTRY(matvec_chain), ENTRY(rmsnorm), ENTRY(axpy),
+static PyMethodDef methods[] = {ENTRY(matvec), ENTRY(matvec_fused), ENTRY(matvec_chain), ENTRY(rmsnorm), ENTRY(axpy),
                                 ENTRY(act_bf16), ENTRY(gemm_prefill), ENTRY(moe_layer), ENTRY(moe_layer_residual), ENTRY(kv_append),
                                 ENTRY(attn_decode), {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pyhost", NULL, -1, methods, NULL, NULL, NULL, NULL};

@@ -61,3 +61,46 @@ def test_package_fails_loudly_when_library_is_missing(monkeypatch):
     monkeypatch.setattr(L, "LIB_PATH", "/nonexistent/libleviathan_cuda.so")
     with pytest.raises(RuntimeError, match="no fallback"):
         L.load()
+
+
+# the arguments each native call takes (csrc/lev_pyhost.c), handles NULL
+HOST_CALLS = {
+    "matvec": (None, None, 0, 16, None, 32, 1, None, 16, -1, 0),
+    "matvec_fused": (None, None, 0, 16, None, 32, 1, 1, None, 1e-6, None, 1.0, None, 16),
+    "matvec_chain": (None, 1, None, 0),
+    "rmsnorm": (None, None, 1, 32, None, 1e-6, None, None),
+    "axpy": (None, 1.0, None, None, 32, None),
+    "act_bf16": (None, None, 32, None),
+    "gemm_prefill": (None, None, None, 16, None, 0),
+    "moe_layer": (None, None, None, 1, 8, None, None, None, 0),
+    "moe_layer_residual": (None, None, None, 1, 8, None, 1.0, None, 0),
+    "kv_append": (None, None, None, None, None, None, None, 1, None, None),
+    "attn_decode": (None, None, None, None, None, None, None, 1, 8, None, 0, 1.0, None),
+}
+
+
+def test_host_layer_native_and_through_ctypes(lib, monkeypatch, tmp_path):
+    """Both forms of the per-token calls take the same arguments; without a file for this interpreter, ctypes serves."""
+    native = L.host()
+    assert os.path.exists(L.HOST_PATH) and sorted(n for n in dir(native) if not n.startswith("_")) == sorted(HOST_CALLS)
+    monkeypatch.setattr(L, "_host", None)
+    monkeypatch.setattr(L, "HOST_PATH", str(tmp_path / "missing.so"))
+    through_ctypes = L.host()
+    for name, args in HOST_CALLS.items():
+        a, b = getattr(native, name)(*args), getattr(through_ctypes, name)(*args)
+        assert a == b and L.STATUS[a] == "badArgument", name
+        for form in (native, through_ctypes):
+            with pytest.raises(TypeError):
+                getattr(form, name)(*args[:-1])
+
+
+def test_build_without_a_compiler_leaves_ctypes(lib, monkeypatch, tmp_path):
+    from leviathan_b200 import build
+
+    path = tmp_path / "_pyhost.so"
+    monkeypatch.setattr(build, "HOST_PATH", str(path))
+    monkeypatch.setenv("CC", str(tmp_path / "no-such-compiler"))
+    assert build.build_library() == build.LIB_PATH and not path.exists()
+    path.write_bytes(b"of another library")
+    os.utime(path, (0, 0))
+    assert build.build_library() == build.LIB_PATH and not path.exists()
