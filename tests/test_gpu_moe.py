@@ -228,7 +228,7 @@ def test_layer_with_folded_residual_gives_the_bits_of_layer_then_axpy(ctx, model
 @pytest.mark.parametrize("tokens", [96, 512])
 def test_prefill_sized_layer_runs_on_the_tensor_cores(ctx, models, tokens):
     """96 tokens x top-8 = 768 pairs and the 512-token batch (4096 pairs): the expert FFN runs as a
-    grouped bf16 dequant-GEMM (tcgen05); routing stays bit-exact, outputs are held to the 2e-2 bar of
+    grouped f16 dequant-GEMM (tcgen05); routing stays bit-exact, outputs are held to the 2e-2 bar of
     tensor-core prefill and reported against 5e-3."""
     m = models["gemma"]
     e, h, i, k = m["dims"]

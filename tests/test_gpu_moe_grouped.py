@@ -132,3 +132,68 @@ def test_resident_experts_only(ctx, first, count):
     assert bool(((y.double() - want).abs() <= bound)[mine].all())
     part.free()
     layer.mw.free()
+
+
+@pytest.mark.parametrize("experts,hidden,inter,top_k,tokens,crowd", [
+    (8, 1056, 96, 2, 600, 0),       # 256-token jobs (over 40 pairs an expert); hidden and inter with half chunks of K and
+    (8, 1056, 96, 2, 600, 590),     # partly filled row tiles; an expert with three jobs, the last ragged
+    (4, 256, 32, 1, 1030, 0),       # one chunk of K in the down product: teams without work
+    (4, 64, 32, 2, 520, 513),       # one chunk in both, a last job of one token
+    (32, 1056, 96, 4, 256, 200),    # 64-token jobs, several of one expert
+    (32, 96, 544, 4, 260, 129),
+    (64, 192, 224, 8, 130, 0),
+])
+def test_jobs_tiles_and_remainders(ctx, experts, hidden, inter, top_k, tokens, crowd):
+    rng = np.random.default_rng(hidden + crowd)
+    layer = Layer(ctx, experts, hidden, inter, hidden + inter + crowd)
+    x = torch.from_numpy(Q.normal(tokens, (tokens, hidden), 1.0)).cuda()
+    idx = routing(rng, tokens, top_k, experts, crowd)
+    want, bound, act, act_b = reference(layer, x, idx)
+    y, a = ctx.moe_experts(layer.mw, x, idx, want_act=True)
+    ctx.synchronize()
+    assert bool(((y.double() - want).abs() <= bound).all()), float(((y.double() - want).abs() / bound).max())
+    assert bool(((a.double() - act).abs() <= act_b).all()), float(((a.double() - act).abs() / act_b).max())
+    assert torch.equal(y, ctx.moe_experts(layer.mw, x, idx))
+    layer.mw.free()
+
+
+def test_rows_of_any_magnitude(ctx):
+    """A row of activations is scaled by a power of two of its own: zeros, far below and above the f16 range, and one with an
+    infinity, whose token alone is not finite."""
+    rng = np.random.default_rng(5)
+    layer = Layer(ctx, 32, 1152, 128, 55)
+    x = torch.from_numpy(Q.normal(56, (256, 1152), 1.0)).cuda()
+    x[3], x[4], x[5], x[6] = 0.0, x[4] * 1e-30, x[5] * 1e9, x[6] * 1e-6
+    x[7, 100] = 3e4
+    x[200, 17] = float("inf")
+    x[201, 1151] = float("nan")
+    idx = routing(rng, 256, 4, 32)
+    y = ctx.moe_experts(layer.mw, x, idx)
+    ctx.synchronize()
+    bad = torch.zeros(256, dtype=torch.bool, device="cuda")
+    bad[[200, 201]] = True
+    assert not bool(torch.isfinite(y[bad]).any())
+    clean = x.clone()
+    clean[bad] = 0.0
+    want, bound, _, _ = reference(layer, clean, idx)
+    assert bool(((y.double() - want).abs() <= bound)[~bad].all())
+    assert bool((y[3] == 0).all())
+    layer.mw.free()
+
+
+def test_scales_beyond_f16_products_take_the_f32_forms(ctx):
+    """A block scale of 65504: d * (q - 8) leaves the f16 range, so the layer keeps to the kernels with f32 scales."""
+    def edit(gu, dn):
+        dn[0:2] = np.array([0xFF, 0x7B], np.uint8)                      # expert 0, row 0, block 0
+        dn[18 * 4 * 10:18 * 4 * 10 + 2] = np.array([0xFF, 0xFB], np.uint8)   # row 10: the negative one
+
+    rng = np.random.default_rng(6)
+    layer = Layer(ctx, 32, 256, 128, 66, edit)
+    x = torch.from_numpy(Q.normal(67, (256, 256), 1.0)).cuda()
+    idx = routing(rng, 256, 4, 32)
+    y = ctx.moe_experts(layer.mw, x, idx)
+    ctx.synchronize()
+    want, bound, _, _ = reference(layer, x, idx)
+    assert bool(torch.isfinite(y).all()) and bool(((y.double() - want).abs() <= bound).all())
+    assert float((y.double() - want).norm() / want.norm()) < 1e-4
+    layer.mw.free()

@@ -99,6 +99,27 @@ def test_norm_prologue_matches_norm_then_matvec(ctx, name, rows, cols, n_cols):
     wh.free()
 
 
+@pytest.mark.parametrize("name,rows,cols", [("q4_k", 48, 256), ("q6_k", 35, 512), ("q4_0", 300, 1056)])
+@pytest.mark.parametrize("n_cols", [1, 2, 4, 5, 8])
+def test_norm_weight_off_a_16_byte_boundary(ctx, name, rows, cols, n_cols):
+    """The one-launch kernel reads the norm weight in 16-byte vectors; other addresses run the steps one by one."""
+    t = H.TYPES[name]
+    w = H.quantized(t, 17, rows, cols)
+    wh, wh2 = ctx.upload(w, t, rows, cols), ctx.upload(w, t, rows, cols)
+    x = dev(Q.normal(18, (n_cols, cols), 1.5).astype(np.float32))
+    buf = dev((1.0 + Q.normal(19, (cols + 1,), 0.1)).astype(np.float32))
+    nw = buf[1:]
+    assert nw.data_ptr() % 16 == 4
+    want = ctx.matvec(wh, ctx.rmsnorm(x, nw.clone(), 1e-6)).cpu().numpy().astype(np.float64).reshape(-1)
+    res = dev(Q.normal(20, (n_cols, rows), 1.0).astype(np.float32))
+    got = ctx.matvec_fused(wh, x, "rmsnorm", nw, 1e-6, residual=res, alpha=2.0).cpu().numpy().reshape(-1)
+    assert O.max_rel_err(got, res.cpu().numpy().astype(np.float64).reshape(-1) + 2.0 * want) < 1e-5
+    for y in ctx.matvec_multi_fused([wh, wh2], x, "rmsnorm", nw, 1e-6):
+        assert O.max_rel_err(y.cpu().numpy().reshape(-1), want) < 1e-5
+    wh.free()
+    wh2.free()
+
+
 @pytest.mark.parametrize("name,rows,inter", [("q4_k", 2816, 2304), ("q6_k", 2816, 2304), ("q4_0", 2816, 704), ("q4_0", 35, 96)])
 @pytest.mark.parametrize("n_cols", [1, 4, 5])
 def test_gelu_prologue_and_residual_epilogue(ctx, name, rows, inter, n_cols):
