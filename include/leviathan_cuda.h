@@ -138,7 +138,8 @@ int lev_cuda_destroy(lev_ctx* ctx);
 const char* lev_last_error(const lev_ctx* ctx);
 int lev_cuda_hardware_profile(lev_ctx* ctx, lev_hw_profile* out);
 /* cuda_stream is a cudaStream_t; NULL restores the context's own stream (pass
- * cudaStreamLegacy, not 0, to name the legacy default stream). */
+ * cudaStreamLegacy, not 0, to name the legacy default stream).  Work buffers belong to the context: the
+ * caller orders its calls on different streams, lev_gemm_prefill and lev_act_bf16 excepted. */
 int lev_cuda_set_stream(lev_ctx* ctx, void* cuda_stream);
 /* waits for the stream; LEV_TIMEOUT if a kernel's bounded wait ran out, LEV_BAD_DIMENSIONS if a
  * cache index lay outside its layout (kernels record these instead of faulting) */
@@ -159,8 +160,8 @@ int lev_weights_upload(lev_ctx* ctx, const void* bytes, size_t n_bytes, int ggml
 int lev_weights_free(lev_ctx* ctx, lev_weights* w);
 int lev_weights_info(const lev_weights* w, int* ggml_type, int64_t* rows, int64_t* cols,
                      size_t* gguf_bytes);
-/* A resident tensor is held twice: in GGUF order (read by lev_dequantize, the plain schedule and the
- * prefill GEMM) and repacked in tile order for the stream schedule (the same bytes, permuted).  A
+/* A resident tensor is held twice: in GGUF order (read by lev_dequantize, the plain schedule and, for activations
+ * off a 16-byte boundary, the prefill GEMM) and repacked in tile order for the stream schedule (the same bytes, permuted).  A
  * decode-only host can release the GGUF-order copy, as the reference keeps one resident buffer per
  * model (Sources/LeviathanCore/Gemma4.swift:2622-2631); the entry points that read it then return
  * LEV_UNSUPPORTED for this tensor. */
@@ -400,8 +401,9 @@ int lev_moe_weights_upload(lev_ctx* ctx, const float* router_w, const uint8_t* g
                            int local_count, int bytes_on_device, lev_moe_weights** out);
 int lev_moe_weights_free(lev_ctx* ctx, lev_moe_weights* w);
 /* lev_weights_release_gguf for both expert tensors of a layer: a decode-only host keeps one copy of the
- * experts (the repacked one).  Calls the tensor-core form would serve (from 512 token-slot pairs on, where the
- * job-list form no longer applies; it reads the GGUF-order bytes) then run on the multi-column stream kernels. */
+ * experts (the repacked one).  It also asks for f32 precision throughout: calls that the tensor-core form would serve
+ * (f16 operands; from 512 token-slot pairs on, where the job-list form no longer applies) then run on the
+ * multi-column stream kernels. */
 int lev_moe_weights_release_gguf(lev_ctx* ctx, lev_moe_weights* w);
 
 /* Router decision for `tokens` rows of x [tokens][hidden]: logits in the

@@ -887,8 +887,8 @@ extern "C" int lev_moe_weights_upload(lev_ctx* ctx, const float* router_w, const
 }
 
 // Drops the GGUF-order copies of the expert tensors.  The decode-sized forms of the layer (below 512 token-slot
-// pairs) read the repacked copies only; the tensor-core form reads the GGUF bytes, so a layer released here
-// runs larger batches through the multi-column stream kernels instead.
+// pairs) read the repacked copies only.  So does the tensor-core form, but in f16 operands: a layer released here
+// keeps f32 precision and runs larger batches through the multi-column stream kernels instead.
 extern "C" int lev_moe_weights_release_gguf(lev_ctx* ctx, lev_moe_weights* w) {
     if (!ctx || !w || !w->gate_up || !w->down) return LEV_BAD_ARGUMENT;
     LEV_TRY(lev_weights_release_gguf(ctx, w->gate_up));
@@ -1089,9 +1089,11 @@ static int experts_dev_impl(lev_ctx* ctx, const lev_moe_weights* w, const float*
     const bool sliced = moe_sliced(ctx, w, pairs, x);
     // prefill-sized calls: grouped dequant-GEMM on the tensor cores (f16 operands, f32 accumulate;
     // the 2e-2 bar of tensor-core prefill applies to this form)
-    // Mid-sized calls (one job per expert and four of its tokens) take the one-launch kernel as far as its tables
-    // allow -- 84 tokens of the 128-expert top-8 shape: 180 us at 64 tokens, 222 at 84, where the grouped GEMM costs a
-    // flat 300 us up to about 128 tokens -- and from 1024 pairs on the GEMM is preferred wherever it applies.
+    // Mid-sized calls (one job per expert and four of its tokens) take the one-launch kernel, whose weights and activations
+    // keep f32 precision, as far as its tables allow, up to 1024 pairs.  That line is about precision, not only about time:
+    // layers of 128 experts (2816 / 704, top-8) take 136 us at 256 pairs, 183 at 512 and 217 at 640 there, 176, 193 and 202
+    // on the GEMM; with fewer experts the GEMM would be the faster one sooner (64 experts, 2048 / 1024: 160 us at 510
+    // pairs against 113; 16 experts, 2048 / 704: 130 at 512 against 71).
     const bool sliced4_early = !sliced && pairs < 1024 && moe_sliced4(ctx, w, pairs, x);
     const int64_t min_pairs = 512;
     const bool tensor = !sliced && !sliced4_early && pairs >= min_pairs && lev_moe_gemm_supported(w);
