@@ -610,8 +610,13 @@ bool dense_plan_tiles(lev_ctx* ctx, const lev_weights* w, int64_t tiles, int n_c
         // columns 49.5 us, 56.6 here; [8192 x 7680] at five 24.3, 27.1 here), Q4_0 (56.4, 53.7 here) and Q6_K are not.
         cap = 200 * 1024;
         warps = tb + 16 * 2 * step <= cap ? 16 : tb + 12 * 2 * step <= cap ? 12 : 8;
-        if (warps == 8 && w->type == LEV_GGML_Q4_K) return false;
         if (tb + 8 * 2 * step > cap) return false;
+        if (warps == 8 && w->type == LEV_GGML_Q4_K) {
+            // unless the other kernel's tables would need their buffer inside a stream capture, where it cannot grow
+            const bool sized = ctx->scratch_bytes[LEV_SCR_XPREP] >= lev_stream_table_bytes(w, n_cols, lev_stream_terms(n_cols), 1, nullptr) + 256;
+            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+            if (sized || cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs == cudaStreamCaptureStatusNone) return false;
+        }
     }
     const int sms = ctx->prop.multiProcessorCount;
     const int grid = (int)(tiles < sms ? tiles : sms);

@@ -1,21 +1,22 @@
 // Grouped dequant-GEMM of the routed MoE at prefill-sized token counts (tcgen05 + TMEM), sm_100a: the Q4_0 weight rows of
 // an expert are the MMA's M (128 per CTA), the tokens routed to it its N (up to 64 or 256 per job).
 //
-// An expert's weights are decoded for a few dozen tokens only, so the decode bounds the kernel (512 tokens of 128 experts,
-// top-8: issue slots 68 %, ALU 61 % used, tensor cores active 18 % of the time), and it is cut to the bone here: operands are f16.  A nibble masked in place under the exponent of 1024 is the f16 number 1024 + q (or
-// 1024 + 16 q), one packed f16 operation makes it q - 8 exactly and one multiplies by the block's f16 scale, so two
-// weights cost three instructions where bf16 through f32 (lev_gemm_pk.cuh) costs five, and the one rounding is to
-// 11 bits instead of 8.  Activation rows are scaled by a power of two so that their largest element lies in
-// [2^14, 2^15): they keep 11 bits wherever they matter (bf16 kept 8), nothing overflows, and the epilogue multiplies
-// the power back.  Experts whose scales could overflow f16 in d * (q - 8) do not take this form.
+// An expert's weights are decoded for a few dozen tokens only, so the decode bounds the kernel (512 tokens of 128
+// experts, top-8: issue slots 68 %, ALU 61 % used, tensor cores active 18 % of the time), and it is cut to the bone
+// here: operands are f16.  A nibble masked in place under the exponent of 1024 is the f16 number 1024 + q (or 1024 +
+// 16 q), one packed f16 operation makes it q - 8 exactly and one multiplies by the block's f16 scale, so two weights
+// cost three instructions where bf16 through f32 (lev_gemm_pk.cuh) costs five, and the one rounding is to 11 bits
+// instead of 8.  Activation rows are scaled by a power of two so that their largest element lies in [2^14, 2^15):
+// they keep 11 bits wherever they matter (bf16 kept 8), nothing overflows, and the epilogue multiplies the power
+// back.  Experts whose scales could overflow f16 in d * (q - 8) do not take this form.
 //
 // The pairs a mask yields are columns (4t, 4t + 2), (16 + 4t, ...), (4t + 1, 4t + 3), ...: the activation rows are
 // stored in that order (k_rows_f16), which leaves the dot product as it is.
 //
-// Roles of the 31 warps as in lev_gemm_pk.cu, with three teams of eight decode warps; tiles come from the device-side job list.  A stage holds one 64-column
-// chunk, or two where jobs are small (then a decode warp fills two chunks per handshake and the MMA warp waits once
-// per eight MMAs).  gate_up tiles interleave 16 gate rows with the 16 up rows that go with them, so gelu(gate) * up is
-// formed in the epilogue by one exchange between half-warps.
+// Roles of the 31 warps as in lev_gemm_pk.cu, with three teams of eight decode warps; tiles come from the device-side
+// job list.  A stage holds one 64-column chunk, or two where jobs are small (then a decode warp fills two chunks per
+// handshake and the MMA warp waits once per eight MMAs).  gate_up tiles interleave 16 gate rows with the 16 up rows
+// that go with them, so gelu(gate) * up is formed in the epilogue by one exchange between half-warps.
 #include "lev_gemm_pk.cuh"
 #include "lev_umma.cuh"
 #include "lev_stream.h"

@@ -393,3 +393,22 @@ def test_route_of_five_to_eight_columns(ctx, name, n_cols, cols, launches):
         assert O.max_rel_err(yw[c].cpu().numpy(), O.matvec_f64(H.TYPES["q6_k"], wide, 48, 12288, xw[c])) < H.REPORT_TOL
     wh.free()
     wwh.free()
+
+
+def test_first_call_of_seven_columns_inside_a_capture():
+    """The two-launch kernel's tables need a buffer that cannot grow there: the one-launch kernel serves the call."""
+    fresh = lev.Context(0)
+    t = H.TYPES["q4_k"]
+    w = H.quantized(t, 65, 160, 5632)
+    x = Q.normal(66, (7, 5632), 1.0)
+    wh, dx, y = fresh.upload(w, t, 160, 5632), torch.from_numpy(x).cuda(), torch.zeros((7, 160), device="cuda")
+    torch.cuda.synchronize()
+    stream, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        fresh.matvec(wh, dx, out=y)
+    g.replay()
+    torch.cuda.synchronize()
+    for c in range(7):
+        assert O.max_rel_err(y[c].cpu().numpy(), O.matvec_f64(t, w, 160, 5632, x[c])) < H.REPORT_TOL
+    wh.free()
+    fresh.close()
